@@ -83,11 +83,11 @@ struct KrFactors {
 // MTTKRP kernels take an explicit device workspace (split-contraction
 // partials), so a captured CUDA graph can own its memory.
 //
-// CUDA-core path (mttkrp_simt.cu): FP32 FMA; with round = 1 (FP16) or 2
+// CUDA-core path (mttkrp_ffma.cu): FP32 FMA; with round = 1 (FP16) or 2
 // (BF16) the operands -- X and each formed KR row -- are rounded first.
-size_t mttkrp_simt_ws_bytes(int order, const long *dims, int mode, long R, int round);
-int mttkrp_simt_rounded(const float *X, int order, const long *dims, const float *const *U,
-                        int mode, long R, float *out, int round, void *ws, cudaStream_t s);
+size_t mttkrp_ffma_ws_bytes(int order, const long *dims, int mode, long R, int round);
+int mttkrp_ffma(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,
+                int round, void *ws, cudaStream_t s);
 // The CUDA-core MTTKRP on FP64 data (FP64 CP-ALS); ws as sized below.
 size_t mttkrp_simt_f64_ws_bytes(int order, const long *dims, int mode, long R);
 int mttkrp_simt_f64(const double *X, int order, const long *dims, const double *const *U, int mode, long R,
@@ -108,6 +108,11 @@ struct MttkrpParts {
 // layout is returned there and `out` is not written.
 int mttkrp_tc(const float *X, int order, const long *dims, const float *const *U, int mode,
               long R, float *out, int precision, void *ws, cudaStream_t s, MttkrpParts *parts = nullptr);
+// The split reduce (mttkrp.cu): out (Q x R, column-major) = the sum of the
+// partials over the splits in FP64, in a fixed order.  Rp = 0: partials
+// [split][r][q]; else [split][q][Rp].  NaN everywhere when *error is set.
+// Launched programmatically behind the kernel that writes the partials.
+int sum_splits(const float *part, int splits, long Q, long R, long Rp, const int *error, float *out, cudaStream_t s);
 // Dispatcher (mttkrp.cu): tensor cores when they apply, else CUDA cores.
 size_t mttkrp_ws_bytes(int order, const long *dims, int mode, long R, int precision);
 int mttkrp_run(const float *X, int order, const long *dims, const float *const *U, int mode,

@@ -5,19 +5,74 @@
 // otherwise the CUDA-core kernel with the same operand rounding
 // (BF16X3/DEFAULT fall back to plain FP32, which is at least as accurate).
 #include "kernels.cuh"
+#include "tc_ptx.cuh"
 
 namespace cud {
 
 namespace {
+
+// A CTA owns 32 consecutive slots of a partial (coalesced reads), each summed
+// by ZL lanes over the splits z = lane, lane + ZL, .. and then in a fixed
+// two-level order.  Bound: the latency of the chain of L2 reads, so the lanes
+// are as many as the splits can feed.
+template <int ZL>
+__global__ void __launch_bounds__(32 * ZL) k_sum_splits(const float *__restrict__ part, int splits, long Q, long R,
+                                                        long Rp, const int *__restrict__ error,
+                                                        float *__restrict__ out) {
+    __shared__ double red[ZL][32];
+    const int o = threadIdx.x & 31, zl = threadIdx.x >> 5;
+    const long e = blockIdx.x * 32L + o;
+    const long n = Q * (Rp ? Rp : R);
+    ptx::griddep_wait();  // the partials
+    double sum = 0.0;
+    if (e < n) {
+#pragma unroll 8
+        for (int z = zl; z < splits; z += ZL) sum += (double)__ldcs(part + (long)z * n + e);
+    }
+    red[zl][o] = sum;
+    __syncthreads();
+    constexpr int G = ZL > 8 ? 4 : 1;  // second-level sums
+    if (zl < G) {
+#pragma unroll
+        for (int k = zl + G; k < ZL; k += G) sum += red[k][o];
+        if (G > 1) red[zl][o] = sum;
+    }
+    if (G > 1) __syncthreads();
+    if (zl == 0 && e < n) {
+#pragma unroll
+        for (int k = 1; k < G; k++) sum += red[k][o];
+        // a CTA whose bounded wait expired left its partial incomplete: the
+        // output becomes NaN so the failure cannot pass for a result
+        if (error && *error) sum = __longlong_as_double(0x7ff8000000000000LL);
+        if (Rp) {
+            const long q = e / Rp, r = e - q * Rp;
+            if (r < R) out[q + Q * r] = (float)sum;
+        } else {
+            out[e] = (float)sum;
+        }
+    }
+}
 int round_mode(int precision) {
     return precision == CUD_PREC_FP16 ? 1 : precision == CUD_PREC_BF16 ? 2 : 0;
 }
 }  // namespace
 
+int sum_splits(const float *part, int splits, long Q, long R, long Rp, const int *error, float *out, cudaStream_t s) {
+    const long ctas = (Q * (Rp ? Rp : R) + 31) / 32;
+    // 32 lanes an output where the splits feed them and the grid is about a
+    // wave of such CTAs (B200, a call: 96^4 R = 32, 294 splits of 96 CTAs 4.4
+    // against 8.1 us; 512^3 R = 64, 73 splits of 1024 CTAs 10.6 against 5.0)
+    const bool wide = splits >= 32 && ctas <= 4L * kNumSMs;
+    PdlLaunch l((unsigned)ctas, wide ? 1024 : 256, 0, s);
+    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, wide ? k_sum_splits<32> : k_sum_splits<8>, part, splits, Q, R, Rp, error, out));
+    CUD_CHECK_LAUNCH("mttkrp reduce");
+    return CUD_OK;
+}
+
 // Sized for both paths, so a call may fall back (e.g. a misaligned X) with
 // the same workspace.
 size_t mttkrp_ws_bytes(int order, const long *dims, int mode, long R, int precision) {
-    size_t b = mttkrp_simt_ws_bytes(order, dims, mode, R, round_mode(precision));
+    size_t b = mttkrp_ffma_ws_bytes(order, dims, mode, R, round_mode(precision));
     size_t t = 0;
     if (precision != CUD_PREC_FP32 && mttkrp_tc_query(order, dims, mode, R, precision, &t) == CUD_OK)
         b = std::max(b, t);
@@ -33,7 +88,7 @@ int mttkrp_run(const float *X, int order, const long *dims, const float *const *
             if (st != CUD_ERR_UNSUPPORTED) return st;
         }
     }
-    return mttkrp_simt_rounded(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
+    return mttkrp_ffma(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
 }
 
 int mttkrp_run_parts(const float *X, int order, const long *dims, const float *const *U, int mode, long R,
@@ -45,7 +100,7 @@ int mttkrp_run_parts(const float *X, int order, const long *dims, const float *c
             if (st != CUD_ERR_UNSUPPORTED) return st;
         }
     }
-    int st = mttkrp_simt_rounded(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
+    int st = mttkrp_ffma(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
     if (st == CUD_OK) *parts = MttkrpParts{out, 0, 1, dims[mode], 1, nullptr};
     return st;
 }

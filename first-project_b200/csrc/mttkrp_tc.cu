@@ -1163,76 +1163,6 @@ __global__ void __launch_bounds__(PB_THREADS, MINB)
     ptx::griddep_launch();
 }
 
-// The same sum with one warp per output (lane l takes z = l, l + 32, ...,
-// then a fixed shuffle tree), for outputs too few to fill the GPU with the
-// 8-lane layout below (96 x 32 outputs at 96^4 rank 32: 96 CTAs of 37
-// sequential loads each).
-__global__ void __launch_bounds__(256) k_sum_tc_partials_w(const float *__restrict__ part, int splits, long Q,
-                                                           long R, long Rp, const int *__restrict__ error,
-                                                           float *__restrict__ out) {
-    ptx::griddep_wait();  // the MTTKRP grid's partials
-    const int lane = threadIdx.x & 31;
-    const long e = blockIdx.x * 8L + (threadIdx.x >> 5);  // q * Rp + r
-    const long n = Q * Rp;
-    if (e >= n) return;  // warp-uniform
-    double sum = 0.0;
-#pragma unroll 4
-    for (int z = lane; z < splits; z += 32) sum += (double)__ldcs(part + (long)z * n + e);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) {
-        const long q = e / Rp, r = e - q * Rp;
-        if (*error) sum = __longlong_as_double(0x7ff8000000000000LL);
-        if (r < R) out[q + Q * r] = (float)sum;
-    }
-}
-
-// Launches the split reduce in the layout that fills the GPU.
-void sum_tc_partials(const float *part, int splits, long Q, long R, long Rp, const int *error, float *out,
-                     cudaStream_t s);
-
-// out[q + Q r] = sum_z part[z][q][r] in FP64, fixed order.  A CTA owns 32
-// consecutive (q, r) slots of the padded partial rows (coalesced reads), each
-// summed by 8 lanes over the splits z = lane, lane + 8, ..., then combined
-// in lane order.
-__global__ void __launch_bounds__(256) k_sum_tc_partials(const float *__restrict__ part, int splits, long Q,
-                                                         long R, long Rp, const int *__restrict__ error,
-                                                         float *__restrict__ out) {
-    __shared__ double red[8][32];
-    ptx::griddep_wait();  // the MTTKRP grid's partials
-    const int o = threadIdx.x & 31, zl = threadIdx.x >> 5;
-    const long e = blockIdx.x * 32L + o;  // q * Rp + r
-    const long n = Q * Rp;
-    double sum = 0.0;
-    if (e < n) {
-#pragma unroll 16
-        for (int z = zl; z < splits; z += 8) sum += (double)__ldcs(part + (long)z * n + e);
-    }
-    red[zl][o] = sum;
-    __syncthreads();
-    if (zl == 0 && e < n) {
-        double t = red[0][o];
-        for (int k = 1; k < 8; k++) t += red[k][o];
-        const long q = e / Rp, r = e - q * Rp;
-        // a CTA whose bounded wait expired left its partial incomplete: the
-        // output becomes NaN so the failure cannot pass for a result
-        if (*error) t = __longlong_as_double(0x7ff8000000000000LL);
-        if (r < R) out[q + Q * r] = (float)t;
-    }
-}
-
-void sum_tc_partials(const float *part, int splits, long Q, long R, long Rp, const int *error, float *out,
-                     cudaStream_t s) {
-    const long n = Q * Rp;
-    if ((n + 31) / 32 < 2L * kNumSMs && splits > 32) {
-        PdlLaunch l((unsigned)((n + 7) / 8), 256, 0, s);
-        cudaLaunchKernelEx(&l.cfg, k_sum_tc_partials_w, part, splits, Q, R, Rp, error, out);
-    } else {
-        PdlLaunch l((unsigned)((n + 31) / 32), 256, 0, s);
-        cudaLaunchKernelEx(&l.cfg, k_sum_tc_partials, part, splits, Q, R, Rp, error, out);
-    }
-}
-
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     // resolved once (thread-safe static initialisation)
     static const PFN_cuTensorMapEncodeTiled_v12000 fn = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
@@ -1536,9 +1466,7 @@ int mttkrp_tc(const float *X, int order, const long *dims, const float *const *U
             *parts = MttkrpParts{a.part, p.Q * a.Rp, a.Rp, 1, (int)p.splits, a.error};
             return CUD_OK;
         }
-        sum_tc_partials(a.part, (int)p.splits, p.Q, R, a.Rp, a.error, out, s);
-        CUD_CHECK_LAUNCH("mttkrp_tc reduce");
-        return CUD_OK;
+        return sum_splits(a.part, (int)p.splits, p.Q, R, a.Rp, a.error, out, s);
     }
     CUD_CHECK(cudaMemsetAsync(a.error, 0, sizeof(int), s));
     // two D buffers + nst A stages of 32 columns, rounded to a power of two
@@ -1562,9 +1490,7 @@ int mttkrp_tc(const float *X, int order, const long *dims, const float *const *U
         *parts = MttkrpParts{a.part, p.Q * a.Rp, a.Rp, 1, (int)p.splits, a.error};
         return CUD_OK;
     }
-    sum_tc_partials(a.part, (int)p.splits, p.Q, R, a.Rp, a.error, out, s);
-    CUD_CHECK_LAUNCH("mttkrp_tc reduce");
-    return CUD_OK;
+    return sum_splits(a.part, (int)p.splits, p.Q, R, a.Rp, a.error, out, s);
 }
 
 }  // namespace cud
