@@ -5,7 +5,7 @@
 // solve) with `typedef double dt` -- as one general-order entry over device
 // pointers, like cud_cp_als.
 //
-// Per mode: the CUDA-core MTTKRP on FP64 data (mttkrp_simt.cu, no
+// Per mode: the FP64 MTTKRP (mttkrp_f64.cu, no
 // Khatri-Rao matrix), V = Hadamard of the other FP64 Grams and its inverse
 // (solve.cu's normal_inverse: Gauss-Jordan with Cholesky's pivots, Jacobi
 // pseudo-inverse fallback), U = M V^-1 and the new factor's Gram.  The fit
@@ -107,9 +107,9 @@ extern "C" int cud_mttkrp_f64(const double *X, int order, const long *dims, cons
         if (m != mode && !U[m]) return set_status(CUD_ERR_INVALID_ARGUMENT);
     }
     int st;
-    void *ws = scratch(kSlotMttkrp, mttkrp_simt_f64_ws_bytes(order, dims, mode, R), &st);
+    void *ws = scratch(kSlotMttkrp, mttkrp_f64_ws_bytes(order, dims, mode, R), &st);
     if (!ws) return set_status(st);
-    return set_status(mttkrp_simt_f64(X, order, dims, U, mode, R, out, ws, as_stream(stream)));
+    return set_status(mttkrp_f64(X, order, dims, U, mode, R, out, ws, as_stream(stream)));
 }
 
 extern "C" int cud_cp_als_f64(const double *X, int order, const long *dims, long R, double *const *U,
@@ -130,7 +130,7 @@ extern "C" int cud_cp_als_f64(const double *X, int order, const long *dims, long
 
     // workspace: MTTKRP partials | M | Grams | Vinv | inverse scratch | dot partials | scalars
     size_t mws = 0;
-    for (int m = 0; m < order; m++) mws = std::max(mws, mttkrp_simt_f64_ws_bytes(order, dims, m, R));
+    for (int m = 0; m < order; m++) mws = std::max(mws, mttkrp_f64_ws_bytes(order, dims, m, R));
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t o_m = up(mws), o_g = o_m + up(8 * (size_t)maxd * R), o_v = o_g + up(8 * (size_t)order * R * R),
                  o_w = o_v + up(8 * (size_t)R * R), o_p = o_w + up(8 * (size_t)2 * R * R + 64),
@@ -161,7 +161,7 @@ extern "C" int cud_cp_als_f64(const double *X, int order, const long *dims, long
     for (int sw = 0; sw < opt.max_sweeps; sw++) {
         for (int mode = 0; mode < order; mode++) {
             void *mw = w;  // MTTKRP partials at the start of the workspace
-            if ((st = mttkrp_simt_f64(X, order, dims, Uc, mode, R, M, mw, s))) return set_status(st);
+            if ((st = mttkrp_f64(X, order, dims, Uc, mode, R, M, mw, s))) return set_status(st);
             NormalArgs na;
             for (int m = 0; m < order; m++) na.G[m] = G + (size_t)m * R * R;
             na.nG = order;
