@@ -1,8 +1,8 @@
-// Strided GEMM on CUDA cores: the workhorse for the Tucker side (mode
-// products, unfolding Grams, reconstructions).  64x64 output tile per CTA,
-// 16-deep contraction slices staged through shared memory, 4x4 register tile
-// per thread; optional split of the contraction with an FP64 reduction.
-// The same kernels run on FP32 and FP64 operands (the FP64 Tucker path).
+// Strided GEMM on CUDA cores: mode products, unfolding Grams and
+// reconstructions, for FP64 operands and for the FP32 shapes that
+// gemm_ffma.cu leaves (short contractions, few tiles).  64x64 output tile per
+// CTA, 16-deep contraction slices staged through shared memory, 4x4 register
+// tile per thread; optional split of the contraction with an FP64 reduction.
 #include "kernels.cuh"
 
 namespace cud {
@@ -204,7 +204,10 @@ int gemm_simt_impl(const GemmDescT<T> &d0, cudaStream_t s) {
     return CUD_OK;
 }
 
-int gemm_simt(const GemmDesc &d, cudaStream_t s) { return gemm_simt_impl<float>(d, s); }
+int gemm_simt(const GemmDesc &d, cudaStream_t s) {
+    const int st = gemm_ffma(d, s);
+    return st == CUD_ERR_UNSUPPORTED ? gemm_simt_impl<float>(d, s) : st;
+}
 
 int gemm_simt_f64(const GemmDesc64 &d, cudaStream_t s) {
     if (d.out_f64) return CUD_ERR_INVALID_ARGUMENT;  // FP64 output is the plain path here

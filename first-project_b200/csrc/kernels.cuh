@@ -28,6 +28,9 @@ struct GemmDescT {
 using GemmDesc = GemmDescT<float>;
 using GemmDesc64 = GemmDescT<double>;
 int gemm_simt(const GemmDesc &d, cudaStream_t s);
+// The FP32 kernel for long contractions over many tiles (gemm_ffma.cu);
+// CUD_ERR_UNSUPPORTED, with nothing launched, where it does not apply.
+int gemm_ffma(const GemmDesc &d, cudaStream_t s);
 int gemm_simt_f64(const GemmDesc64 &d, cudaStream_t s);  // FP64 operands and output
 
 // Residual/norm helper (elementwise.cu).  Synchronises the stream.
