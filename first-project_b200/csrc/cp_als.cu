@@ -134,7 +134,7 @@ int enqueue_sweep_fused(cud_cp_plan_s *p, cudaStream_t s, bool join_end) {
     CUD_CHECK(cudaEventRecord(p->ev_join, p->side));
     for (int n = 0; n < N; n++) {
         MttkrpParts parts;
-        st = mttkrp_run_parts(p->X, N, p->dims, (const float *const *)p->U, n, R, p->Mraw, p->opt.precision, p->ws,
+        st = mttkrp_sweep_run(p->X, N, p->dims, (const float *const *)p->U, n, R, p->Mraw, p->opt.precision, p->ws,
                               s, &parts);
         if (st) return st;
         CUD_CHECK(cudaStreamWaitEvent(s, p->ev_join, 0));
@@ -199,7 +199,7 @@ int enqueue_sweep(cud_cp_plan_s *p, cudaStream_t s) {
         na.fallbacks = p->fallbacks;
         if ((st = normal_inverse(na, p->side))) return st;
         CUD_CHECK(cudaEventRecord(p->ev_join, p->side));
-        st = mttkrp_run(p->X, p->order, p->dims, (const float *const *)p->U, n, R, p->M,
+        st = mttkrp_sweep_run(p->X, p->order, p->dims, (const float *const *)p->U, n, R, p->M,
                         p->opt.precision, p->ws, s);
         if (st) return st;
         CUD_CHECK(cudaStreamWaitEvent(s, p->ev_join, 0));
@@ -484,7 +484,7 @@ extern "C" int cud_cp_plan_create(const float *X, int order, const long *dims, l
         maxd = std::max(maxd, dims[m]);
         total *= dims[m];
     }
-    for (int m = 0; m < order; m++) wsb = std::max(wsb, mttkrp_ws_bytes(order, dims, m, R, opt.precision));
+    for (int m = 0; m < order; m++) wsb = std::max(wsb, mttkrp_sweep_ws_bytes(order, dims, m, R, opt.precision));
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     size_t off_M = 0;
     size_t off_Mr = off_M + up(sizeof(float) * maxd * R);

@@ -120,11 +120,17 @@ int sum_splits(const float *part, int splits, long Q, long R, long Rp, const int
 size_t mttkrp_ws_bytes(int order, const long *dims, int mode, long R, int precision);
 int mttkrp_run(const float *X, int order, const long *dims, const float *const *U, int mode,
                long R, float *out, int precision, void *ws, cudaStream_t s);
-// As mttkrp_run, for a consumer that sums the split partials itself: a
-// tensor-core MTTKRP returns its partials in *parts (out not written); any
-// other path writes out and describes it as one column-major split.
-int mttkrp_run_parts(const float *X, int order, const long *dims, const float *const *U, int mode,
-                     long R, float *out, int precision, void *ws, cudaStream_t s, MttkrpParts *parts);
+// The same inside a CP-ALS plan's sweeps, whose CUDA-core kernel is
+// mttkrp_simt.cu's; with `parts`, for a consumer that sums the split partials
+// itself: a tensor-core MTTKRP returns its partials in *parts (out not
+// written); any other path writes out and describes it as one column-major
+// split.
+size_t mttkrp_sweep_ws_bytes(int order, const long *dims, int mode, long R, int precision);
+int mttkrp_sweep_run(const float *X, int order, const long *dims, const float *const *U, int mode, long R,
+                     float *out, int precision, void *ws, cudaStream_t s, MttkrpParts *parts = nullptr);
+size_t mttkrp_simt_ws_bytes(int order, const long *dims, int mode, long R, int round);
+int mttkrp_simt_rounded(const float *X, int order, const long *dims, const float *const *U, int mode, long R,
+                        float *out, int round, void *ws, cudaStream_t s);
 
 // Exact CP residual pieces (residual.cu, residual_tc.cu): per-CTA partial
 // pairs summed in a fixed order into out[0..1]; the tensor-core residual

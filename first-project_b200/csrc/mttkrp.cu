@@ -1,9 +1,11 @@
 // MTTKRP dispatch and the public MTTKRP entry points.
 //
-// CUD_PREC_FP32 runs the CUDA-core kernel; every other precision runs the
+// CUD_PREC_FP32 runs a CUDA-core kernel; every other precision runs the
 // tcgen05 tensor-core kernel where it applies (shape, alignment, rank) and
 // otherwise the CUDA-core kernel with the same operand rounding
 // (BF16X3/DEFAULT fall back to plain FP32, which is at least as accurate).
+// The CUDA-core kernel of the entry points is mttkrp_ffma.cu's; a CP-ALS
+// plan's sweeps keep mttkrp_simt.cu's (see there).
 #include "kernels.cuh"
 #include "tc_ptx.cuh"
 
@@ -91,7 +93,15 @@ int mttkrp_run(const float *X, int order, const long *dims, const float *const *
     return mttkrp_ffma(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
 }
 
-int mttkrp_run_parts(const float *X, int order, const long *dims, const float *const *U, int mode, long R,
+size_t mttkrp_sweep_ws_bytes(int order, const long *dims, int mode, long R, int precision) {
+    size_t b = mttkrp_simt_ws_bytes(order, dims, mode, R, round_mode(precision));
+    size_t t = 0;
+    if (precision != CUD_PREC_FP32 && mttkrp_tc_query(order, dims, mode, R, precision, &t) == CUD_OK)
+        b = std::max(b, t);
+    return b;
+}
+
+int mttkrp_sweep_run(const float *X, int order, const long *dims, const float *const *U, int mode, long R,
                      float *out, int precision, void *ws, cudaStream_t s, MttkrpParts *parts) {
     if (precision != CUD_PREC_FP32) {
         size_t b = 0;
@@ -100,8 +110,8 @@ int mttkrp_run_parts(const float *X, int order, const long *dims, const float *c
             if (st != CUD_ERR_UNSUPPORTED) return st;
         }
     }
-    int st = mttkrp_ffma(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
-    if (st == CUD_OK) *parts = MttkrpParts{out, 0, 1, dims[mode], 1, nullptr};
+    int st = mttkrp_simt_rounded(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
+    if (st == CUD_OK && parts) *parts = MttkrpParts{out, 0, 1, dims[mode], 1, nullptr};
     return st;
 }
 
