@@ -2,18 +2,19 @@
 // shape and rank, one persistent kernel launch per ALS sweep for the whole
 // batch (sized for 4096 tensors with dims in [16, 96] and ranks in [4, 16]).
 //
-// Each CTA pulls tensors from a work queue (largest first) and runs one full
-// sweep of that tensor on its own, everything on-chip except X:
+// CTAs -- clusters of 2 to 8 of them where the tensors are too few to fill the
+// GPU -- pull tensors from a work queue (largest first) and run one full sweep
+// of that tensor, everything on-chip except X:
 //   * the three factor matrices live in shared memory (<= 96 x 16 each,
 //     row-major with the ranks padded to 16 with zeros);
-//   * each MTTKRP reads X straight from global memory into registers with
-//     the lanes of a warp along the tensor's contiguous index i (one
-//     coalesced 128-byte request per load) and contracts it against factor
-//     rows broadcast from shared memory (the ranks are too small for tensor
+//   * each MTTKRP streams X by cp.async through a ring per warp, the lanes
+//     along the tensor's contiguous index i (one coalesced 128-byte request
+//     per warp and copy), and contracts it against factor rows broadcast from
+//     shared memory in packed FP32 FMAs (the ranks are too small for tensor
 //     cores to pay); mode 1 keeps each lane's own row of M, modes 2 and 3
 //     sum the lanes' terms by a recursive-halving shuffle (mttkrp_lanes);
 //   * the R x R normal equations (Hadamard of the FP64 Grams) are inverted
-//     by Gauss-Jordan in shared memory (FP64), with a tiny diagonal shift
+//     by Gauss-Jordan (FP64, a cell per thread), with a tiny diagonal shift
 //     retried when a pivot is not positive;
 //   * the fit comes from ||X||^2 - 2 <M_3, C> + sum prod G (FP64), per
 //     tensor; a tensor whose fit changed by less than `tol` is marked
@@ -23,6 +24,8 @@
 // sweep limit.  The CTA size and the CTAs per SM come from a small autotuner
 // (batched_tune) that times two sweeps per candidate on the batch itself and
 // caches the winner per batch shape class.
+#include <cooperative_groups.h>
+
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -30,21 +33,18 @@
 #include <algorithm>
 
 #include "kernels.cuh"
+#include "tc_ptx.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace cud {
 
 namespace {
 
-// Inner indices whose X loads are issued together (x2 outer indices): 8
-// took the 4096-tensor batch from 0.241 s to 0.217 s against 4; 16 spilled
-// and was slower.
-#ifndef CUD_BATCH_UNROLL
-#define CUD_BATCH_UNROLL 8
-#endif
-
 constexpr int BMAXD = 96;    // largest mode size handled (smem sizing)
 constexpr int BMAXR = 16;    // largest rank handled
 constexpr int RS = BMAXR;    // row stride of factors and results in shared memory (ranks padded)
+constexpr int NORM_PARTS = 8;  // CTAs that share a tensor's norm
 
 struct TensorMeta {
     long xoff;          // offset of X (elements) in the packed tensor buffer
@@ -53,7 +53,7 @@ struct TensorMeta {
     int R;
     int done;
     int sweeps;
-    double normx2;
+    double normp[NORM_PARTS];  // ||X||^2 by parts of the tensor
     double fit, fit_prev;
     double target;      // stop once fit >= target (<= 0: no target)
     double G[3][BMAXR * BMAXR];  // factor Grams (FP64)
@@ -67,38 +67,80 @@ struct BatchArgs {
     float *U;
     unsigned *queue;    // work counter, zero at kernel start
     int *ndone;         // tensors marked converged so far
+    int *error;         // set by a wait that ran out
     int max_sweeps;
     double tol;
     int *fallbacks;
 };
 
 // Shared memory of a CTA of NW warps: the factors and the MTTKRP result
-// row-major (rank contiguous, ranks padded to RS with zeros), and the
-// partial results of the (at most three) 32-row chunks of modes 2 and 3.
+// row-major (rank contiguous, ranks padded to RS), and the partial results of
+// the (at most three) 32-row chunks of modes 2 and 3.
 constexpr int MAXCHUNK = (BMAXD + 31) / 32;
+// Outer and inner indices of X per group of the MTTKRP, and groups in flight.
+constexpr int NO = 4, UN = 4, RING = 4;
 
-template <int NW>
+template <int NW, int CL>
 struct BatchSmem {
-    float F[3][BMAXD * RS];
-    float M[BMAXD * RS];
+    float F[3][BMAXD * RS];                     // rows to a multiple of 4, the last ones zero
+    union {
+        struct {
+            float M[BMAXD * RS];                // this CTA's rows
+            float Mg[CL > 1 ? BMAXD * RS : 4];  // the whole result, gathered from the cluster
+        };
+        float mail[CL > 1 ? NW : 1][BMAXR][32]; // mode 0, before the gather: the sums from the CTA before
+    };
     float Mp[MAXCHUNK][BMAXD * RS];
-    double V[BMAXR * BMAXR];         // normal matrix / its inverse
-    double rowk[BMAXR], colk[BMAXR];
-    double red[32];
+    double G[3][BMAXR * BMAXR];                 // factor Grams (R x R, column-major)
+    double V[BMAXR * BMAXR];                    // inverse of the normal matrix, row-major with stride RS
+    double row[2][BMAXR], col[2][BMAXR], inv[2];
+    double red[2 * NW];
+    double diag[BMAXR];
     int tensor;
-    int fail;
+    float ring[NW][RING][NO * UN * 32];         // X on its way: each lane its own values
+    uint64_t mail_full[NW];
 };
+
+static_assert(2 * (sizeof(BatchSmem<6, 8>) + 1024) <= 228 * 1024, "two CTAs an SM");
 
 template <int NT, class Smem>
 __device__ void load_factors(Smem &sm, const BatchArgs &a, const TensorMeta &t) {
     for (int m = 0; m < 3; m++) {
         const float *src = a.U + t.uoff[m];
         const int I = t.dims[m];
-        for (int e = threadIdx.x; e < I * RS; e += NT) {
+        for (int e = threadIdx.x; e < (I + 3) / 4 * 4 * RS; e += NT) {
             const int i = e / RS, r = e - i * RS;
-            sm.F[m][e] = (r < t.R) ? src[i + I * r] : 0.f;
+            sm.F[m][e] = (r < t.R && i < I) ? src[i + I * r] : 0.f;
         }
+        for (int e = threadIdx.x; e < t.R * t.R; e += NT) sm.G[m][e] = t.G[m][e];
     }
+}
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 dup2(float x) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
+    return v;
+}
+__device__ __forceinline__ void fma2(f32x2 &c, f32x2 a, f32x2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+// D (8 x 8) += A (8 x 4) B (4 x 8) in FP64: lane l holds A[l / 4][l % 4],
+// B[l % 4][l / 4] and D[l / 4][2 (l % 4)], D[l / 4][2 (l % 4) + 1].
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
 }
 
 // Sum of v[0..RP) over the warp's 32 lanes by recursive halving (levels
@@ -126,130 +168,216 @@ __device__ __forceinline__ float lane_sum(float (&v)[RP], int lane) {
     return s;
 }
 
-// M (row-major, I_mode x RS) = MTTKRP of mode `mode`, factors in shared
-// memory.  The lanes of a warp run along i, the tensor's contiguous index
-// (32 rows per warp, ceil(I / 32) warps per row chunk), so every load of X
-// is one coalesced 128-byte request and goes straight into registers; the
-// warps of a chunk split the outer index into contiguous ranges:
+// sm.M (row-major, RS) = this CTA's share of the MTTKRP of mode `mode`,
+// factors in shared memory.  The lanes of a warp run along i, the tensor's
+// contiguous index (32 rows per warp, ceil(I / 32) warps per row chunk), so
+// every load of X is one coalesced 128-byte request and goes straight into
+// registers; the cluster's CTAs, and the warps of a chunk within a CTA, split
+// the outer index:
 //   mode 0: M[i, :] = sum_k C[k, :] * sum_j X[i, j, k] B[j, :]
 //           (outer k, inner j; the lane's own row, no cross-lane sum)
 //   mode 1: M[j, :] = sum_i A[i, :] * sum_k X[i, j, k] C[k, :]
 //   mode 2: M[k, :] = sum_i A[i, :] * sum_j X[i, j, k] B[j, :]
 //           (outer j or k; the lanes' terms summed by lane_sum)
-// Two outer indices at a time, four inner ones unrolled: eight loads in
-// flight per lane, and each broadcast factor row (RP/4 16-byte shared
-// loads) feeds 2 RP FMAs.  (Issuing the next group's loads ahead of the
-// current group's FMAs raised the registers to 166 and measured slower:
-// 0.314 s against 0.255 s for the bench batch; L2 prefetches of the
-// outer pair after next -- bulk for the contiguous slices of modes 1 and 3,
-// per line for mode 2 -- cut the long-scoreboard stalls but measured slower
-// too: 1.58 against 1.38 ms for one sweep of 512 tensors.)  Partials of the warps (mode 0: per outer range;
-// modes 1, 2: per row chunk) are combined in a fixed order.  RP = the rank
-// rounded up to 4, 8 or 16; the padding ranks are zero.
-template <int NW, int RP>
-__device__ void mttkrp_lanes(BatchSmem<NW> &sm, const BatchArgs &a, const TensorMeta &t, int mode) {
+// X comes NO outer and UN inner indices at a time (zeros past the ends), by
+// cp.async into a ring that only the copying lane reads: RING - 1 groups in
+// flight without registers.  (Loaded to registers, the warps waited for DRAM
+// most of the time: long scoreboard 4.2 stalls an issue.)  In mode 0 a warp's
+// rows are summed over its range of k in k's order whatever the cluster: the
+// CTAs take the range's groups of NO in turn and hand the sums on through
+// distributed shared memory, so results do not depend on the launch shape.  Each broadcast factor row (RP registers, which cost the SM's shared
+// memory a clock each) feeds NO RP multiply-adds (NO RP / 4 clocks), so NO =
+// 4 balances the two; they are packed pairs of ranks (fma.rn.f32x2).  With
+// NO = 2 the kernel was bound by the factor rows' loads.  Partials of the
+// warps (mode 0: per outer range; modes 1, 2: per row chunk) are combined in
+// a fixed order.  RP = the rank rounded up to 4, 8 or 16; the padding ranks
+// of the factors are zero.
+template <int RP, int NW, int CL>
+__device__ void mttkrp_lanes(BatchSmem<NW, CL> &sm, cg::cluster_group &cl, const BatchArgs &a, const TensorMeta &t,
+                             int mode, int rank, uint32_t &mails) {
+    constexpr int H = RP / 2;
     const int I = t.dims[0], J = t.dims[1], K = t.dims[2];
-    const float *X = a.X + t.xoff;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int LI = (I + 31) >> 5;
     const int NG = NW / LI;
     const int ic = warp % LI, g = warp / LI;
     const int i = ic * 32 + lane;
     const bool valid = i < I;
-    const long IJ = (long)I * J;
+    const int IJ = I * J;
     const int O = (mode == 1) ? J : K;        // outer index
     const int Nn = (mode == 1) ? K : J;       // inner index
-    const long so = (mode == 1) ? I : IJ;     // X strides of the outer and inner index
-    const long sn = (mode == 1) ? IJ : I;
+    const int so = (mode == 1) ? I : IJ;      // X strides of the outer and inner index
+    const int sn = (mode == 1) ? IJ : I;
     const float *Vf = (mode == 1) ? sm.F[2] : sm.F[1];  // the inner index's factor rows
-    const int o0 = (g < NG) ? (int)((long)O * g / NG) : O;
-    const int o1 = (g < NG) ? (int)((long)O * (g + 1) / NG) : O;
-    float acc[RP];
+    // this warp's outer range: of the CTA's share, or (mode 0) of the whole,
+    // in groups of NO of which every CL-th is this CTA's
+    const bool turns = CL > 1 && mode == 0;
+    const int c0 = turns ? 0 : O * rank / CL, c1 = turns ? O : O * (rank + 1) / CL;
+    const int begin = (g < NG) ? c0 + (c1 - c0) * g / NG : c1;
+    const int o0 = begin + (turns ? rank * NO : 0);
+    const int o1 = (g < NG) ? c0 + (c1 - c0) * (g + 1) / NG : c1;
+    const int ostep = turns ? CL * NO : NO;
+    f32x2 acc[H];
 #pragma unroll
-    for (int r = 0; r < RP; r++) acc[r] = 0.f;
-    const float *xi = X + (valid ? i : 0);
-    for (int o = o0; o < o1; o += 2) {
-        const bool two = o + 1 < o1;
-        float t0[RP], t1[RP];
+    for (int r = 0; r < H; r++) acc[r] = 0;
+    // the copies run RING - 1 groups ahead: position (po, pn)
+    int po = o0, pn = 0, fill = 0, slot = 0;
+    const float *px = a.X + t.xoff + (valid ? i : 0) + (long)so * o0;
+    const uint32_t ring = smem_u32(&sm.ring[warp][0][lane]);
+    const int size = valid ? 4 : 0;  // lanes past I copy zeros (and read nothing)
+    auto copy = [&]() {
+        if (po < o1) {
+            const uint32_t d = ring + (uint32_t)fill * (NO * UN * 128u);
+            const int lo = o1 - po, ln = Nn - pn;
+            const float *pk = px;
+            if (lo >= NO && ln >= UN) {
 #pragma unroll
-        for (int r = 0; r < RP; r++) { t0[r] = 0.f; t1[r] = 0.f; }
-        const float *x0 = xi + so * o;
-        const float *x1 = xi + so * (two ? o + 1 : o);
-        const bool l0 = valid, l1 = valid && two;
-        int n = 0;
-        for (; n + CUD_BATCH_UNROLL <= Nn; n += CUD_BATCH_UNROLL) {
-            float xa[CUD_BATCH_UNROLL], xb[CUD_BATCH_UNROLL];
+                for (int k = 0; k < UN; k++, pk += sn) {
+                    const float *pu = pk;
 #pragma unroll
-            for (int u = 0; u < CUD_BATCH_UNROLL; u++) {
-                xa[u] = l0 ? __ldg(x0 + sn * (n + u)) : 0.f;
-                xb[u] = l1 ? __ldg(x1 + sn * (n + u)) : 0.f;
+                    for (int u = 0; u < NO; u++, pu += so)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + (k * NO + u) * 128u),
+                                     "l"(pu), "r"(size));
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < UN; k++)
+#pragma unroll
+                    for (int u = 0; u < NO; u++) {
+                        const bool ok = u < lo && k < ln;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + (k * NO + u) * 128u),
+                                     "l"(ok ? pk + (u * so + k * sn) : a.X), "r"(ok ? size : 0));
+                    }
             }
+            pn += UN;
+            px += UN * sn;
+            if (pn >= Nn) {
+                px += ostep * so - pn * sn;
+                pn = 0;
+                po += ostep;
+            }
+        }
+        asm volatile("cp.async.commit_group;");
+        fill = fill + 1 == RING ? 0 : fill + 1;
+    };
+#pragma unroll 1
+    for (int k = 0; k < RING - 1; k++) copy();
+    for (int o = o0; o < o1; o += ostep) {
+        f32x2 tt[NO][H];
 #pragma unroll
-            for (int u = 0; u < CUD_BATCH_UNROLL; u++) {
-                const float *vr = Vf + (n + u) * RS;
+        for (int u = 0; u < NO; u++)
 #pragma unroll
-                for (int r4 = 0; r4 < RP; r4 += 4) {
-                    const float4 v = *reinterpret_cast<const float4 *>(vr + r4);
-                    t0[r4 + 0] = fmaf(xa[u], v.x, t0[r4 + 0]); t1[r4 + 0] = fmaf(xb[u], v.x, t1[r4 + 0]);
-                    t0[r4 + 1] = fmaf(xa[u], v.y, t0[r4 + 1]); t1[r4 + 1] = fmaf(xb[u], v.y, t1[r4 + 1]);
-                    t0[r4 + 2] = fmaf(xa[u], v.z, t0[r4 + 2]); t1[r4 + 2] = fmaf(xb[u], v.z, t1[r4 + 2]);
-                    t0[r4 + 3] = fmaf(xa[u], v.w, t0[r4 + 3]); t1[r4 + 3] = fmaf(xb[u], v.w, t1[r4 + 3]);
+            for (int r = 0; r < H; r++) tt[u][r] = 0;
+#pragma unroll 1
+        for (int n = 0; n < Nn; n += UN) {
+            copy();  // into the slot read a group ago
+            asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
+            const float *xs = &sm.ring[warp][slot][lane];
+            slot = slot + 1 == RING ? 0 : slot + 1;
+            float x[UN][NO];
+#pragma unroll
+            for (int k = 0; k < UN; k++)
+#pragma unroll
+                for (int u = 0; u < NO; u++) x[k][u] = xs[(k * NO + u) * 32];
+#pragma unroll
+            for (int k = 0; k < UN; k++) {
+                const ulonglong2 *vr = reinterpret_cast<const ulonglong2 *>(Vf + (n + k) * RS);
+                f32x2 xx[NO];
+#pragma unroll
+                for (int u = 0; u < NO; u++) xx[u] = dup2(x[k][u]);
+#pragma unroll
+                for (int r = 0; r < H; r += 2) {
+                    const ulonglong2 v = vr[r / 2];
+#pragma unroll
+                    for (int u = 0; u < NO; u++) {
+                        fma2(tt[u][r], xx[u], v.x);
+                        fma2(tt[u][r + 1], xx[u], v.y);
+                    }
                 }
             }
         }
-        for (; n < Nn; n++) {
-            const float xa = l0 ? __ldg(x0 + sn * n) : 0.f;
-            const float xb = l1 ? __ldg(x1 + sn * n) : 0.f;
-            const float *vr = Vf + n * RS;
-#pragma unroll
-            for (int r4 = 0; r4 < RP; r4 += 4) {
-                const float4 v = *reinterpret_cast<const float4 *>(vr + r4);
-                t0[r4 + 0] = fmaf(xa, v.x, t0[r4 + 0]); t1[r4 + 0] = fmaf(xb, v.x, t1[r4 + 0]);
-                t0[r4 + 1] = fmaf(xa, v.y, t0[r4 + 1]); t1[r4 + 1] = fmaf(xb, v.y, t1[r4 + 1]);
-                t0[r4 + 2] = fmaf(xa, v.z, t0[r4 + 2]); t1[r4 + 2] = fmaf(xb, v.z, t1[r4 + 2]);
-                t0[r4 + 3] = fmaf(xa, v.w, t0[r4 + 3]); t1[r4 + 3] = fmaf(xb, v.w, t1[r4 + 3]);
-            }
-        }
         if (mode == 0) {
-            const float *c0 = sm.F[2] + o * RS;
-            const float *c1 = sm.F[2] + (two ? o + 1 : o) * RS;
+            if (turns && o > begin) {
+                // the sums so far, from the CTA that had the group before
+                if (!ptx::mbar_wait_cluster(&sm.mail_full[warp], mails & 1)) *a.error = 1;
+                mails++;
 #pragma unroll
-            for (int r4 = 0; r4 < RP; r4 += 4) {
-                const float4 u = *reinterpret_cast<const float4 *>(c0 + r4);
-                const float4 w = *reinterpret_cast<const float4 *>(c1 + r4);
-                acc[r4 + 0] = fmaf(t1[r4 + 0], w.x, fmaf(t0[r4 + 0], u.x, acc[r4 + 0]));
-                acc[r4 + 1] = fmaf(t1[r4 + 1], w.y, fmaf(t0[r4 + 1], u.y, acc[r4 + 1]));
-                acc[r4 + 2] = fmaf(t1[r4 + 2], w.z, fmaf(t0[r4 + 2], u.z, acc[r4 + 2]));
-                acc[r4 + 3] = fmaf(t1[r4 + 3], w.w, fmaf(t0[r4 + 3], u.w, acc[r4 + 3]));
+                for (int r = 0; r < H; r++) acc[r] = pack2(sm.mail[warp][2 * r][lane], sm.mail[warp][2 * r + 1][lane]);
+            }
+#pragma unroll
+            for (int u = 0; u < NO; u++) {
+                if (o + u >= o1) continue;  // warp-uniform
+                const ulonglong2 *c = reinterpret_cast<const ulonglong2 *>(sm.F[2] + (o + u) * RS);
+#pragma unroll
+                for (int r = 0; r < H; r += 2) {
+                    const ulonglong2 w = c[r / 2];
+                    fma2(acc[r], tt[u][r], w.x);
+                    fma2(acc[r + 1], tt[u][r + 1], w.y);
+                }
+            }
+            if (turns && o + NO < o1) {
+                const int next = rank + 1 == CL ? 0 : rank + 1;
+                float *to = cl.map_shared_rank(&sm.mail[warp][0][lane], next);
+#pragma unroll
+                for (int r = 0; r < H; r++) {
+                    const float2 v = unpack2(acc[r]);
+                    to[64 * r] = v.x;
+                    to[64 * r + 32] = v.y;
+                }
+                ptx::fence_cluster();  // every lane's writes, before lane 0's arrive
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive_cluster(&sm.mail_full[warp], next);
             }
         } else {
             // the lane's terms A[i, :] * t, summed over the lanes (rows i)
             const float *ar = sm.F[0] + (valid ? i : 0) * RS;
 #pragma unroll
-            for (int r4 = 0; r4 < RP; r4 += 4) {
-                const float4 u = *reinterpret_cast<const float4 *>(ar + r4);
-                t0[r4 + 0] *= u.x; t0[r4 + 1] *= u.y; t0[r4 + 2] *= u.z; t0[r4 + 3] *= u.w;
-                t1[r4 + 0] *= u.x; t1[r4 + 1] *= u.y; t1[r4 + 2] *= u.z; t1[r4 + 3] *= u.w;
-            }
-            const float s0 = lane_sum<RP>(t0, lane);
-            const float s1 = lane_sum<RP>(t1, lane);
-            constexpr int SH = (RP == 16) ? 1 : (RP == 8) ? 2 : 3;
-            if ((lane & ((1 << SH) - 1)) == 0) {
-                const int r = lane >> SH;
-                sm.Mp[ic][o * RS + r] = s0;
-                if (two) sm.Mp[ic][(o + 1) * RS + r] = s1;
+            for (int u = 0; u < NO; u++) {
+                if (o + u >= o1) continue;  // warp-uniform
+                float f[RP];
+#pragma unroll
+                for (int r = 0; r < RP; r += 2) {
+                    const float2 v = unpack2(tt[u][r / 2]);
+                    f[r] = v.x * ar[r];
+                    f[r + 1] = v.y * ar[r + 1];
+                }
+                const float s = lane_sum<RP>(f, lane);
+                constexpr int SH = (RP == 16) ? 1 : (RP == 8) ? 2 : 3;
+                if ((lane & ((1 << SH) - 1)) == 0) sm.Mp[ic][(o + u) * RS + (lane >> SH)] = s;
             }
         }
+    }
+    if (turns) {
+        // the range's last CTA (the first, if the range is empty) leaves the
+        // sums with every CTA: rows of group g at g LI 32
+        const int groups = (o1 - begin + NO - 1) / NO;
+        if (g < NG && rank == (groups > 0 ? (groups - 1) % CL : 0)) {
+            for (int c = 0; c < CL; c++) {
+                float4 *to = reinterpret_cast<float4 *>(cl.map_shared_rank(&sm.Mp[0][0], c) + ((g * LI + ic) * 32 + lane) * RS);
+#pragma unroll
+                for (int r = 0; r < RP; r += 4) {
+                    const float2 p = unpack2(acc[r / 2]), q = unpack2(acc[r / 2 + 1]);
+                    to[r / 4] = make_float4(p.x, p.y, q.x, q.y);
+                }
+            }
+        }
+        return;
     }
     if (mode == 0) {
         // the groups' rows added into M in group order, one group per
         // barrier (deterministic, one buffer)
         for (int gg = 0; gg < NG; gg++) {
             if (g == gg && valid) {
+                float4 *m = reinterpret_cast<float4 *>(&sm.M[i * RS]);
 #pragma unroll
-                for (int r = 0; r < RP; r++) {
-                    float *m = &sm.M[i * RS + r];
-                    *m = (gg == 0) ? acc[r] : *m + acc[r];
+                for (int r = 0; r < RP; r += 4) {
+                    const float2 p = unpack2(acc[r / 2]), q = unpack2(acc[r / 2 + 1]);
+                    float4 v = make_float4(p.x, p.y, q.x, q.y);
+                    if (gg) {
+                        const float4 w = m[r / 4];
+                        v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+                    }
+                    m[r / 4] = v;
                 }
             }
             __syncthreads();
@@ -257,8 +385,7 @@ __device__ void mttkrp_lanes(BatchSmem<NW> &sm, const BatchArgs &a, const Tensor
         return;
     }
     __syncthreads();
-    const int Q = t.dims[mode];
-    for (int e = threadIdx.x; e < Q * RS; e += NW * 32) {
+    for (int e = c0 * RS + threadIdx.x; e < c1 * RS; e += NW * 32) {
         if ((e & (RS - 1)) >= RP) continue;  // padding ranks: never read
         float v = 0.f;
         for (int p = 0; p < LI; p++) v += sm.Mp[p][e];
@@ -267,76 +394,157 @@ __device__ void mttkrp_lanes(BatchSmem<NW> &sm, const BatchArgs &a, const Tensor
     __syncthreads();
 }
 
-// V = Hadamard of the Grams other than `mode`; V <- V^-1 (Gauss-Jordan).
-// Leaves sm.fail set when both attempts met a non-positive pivot (V is then
-// not an inverse and the caller keeps the old factor).
-template <int NT, class Smem>
-__device__ void normal_inverse_small(Smem &sm, const BatchArgs &a, const TensorMeta &t, int mode) {
-    const int R = t.R;
-    for (int attempt = 0; attempt < 2; attempt++) {
-        for (int e = threadIdx.x; e < R * R; e += NT) {
-            double v = 1.0;
-            for (int m = 0; m < 3; m++)
-                if (m != mode) v *= t.G[m][e];
-            sm.V[e] = v;
-        }
-        if (threadIdx.x == 0) sm.fail = 0;
-        __syncthreads();
-        double maxdiag = 0.0;
-        for (int j = 0; j < R; j++) maxdiag = fmax(maxdiag, fabs(sm.V[j + R * j]));
-        if (attempt == 1) {
-            __syncthreads();
-            for (int j = threadIdx.x; j < R; j += NT) sm.V[j + R * j] += 1e-10 * maxdiag + 1e-300;
-            __syncthreads();
-        }
-        for (int k = 0; k < R; k++) {
-            const double piv = sm.V[k + R * k];
-            if (!(piv > 1e-14 * maxdiag) || !isfinite(piv)) {
-                if (threadIdx.x == 0) sm.fail = 1;
-                break;
+// The whole M, from the cluster's CTAs, into sm.Mg: mode 0 adds the groups'
+// sums, which every CTA holds, in group order; the others take each row from
+// its CTA.
+template <int NW, int CL>
+__device__ void gather(BatchSmem<NW, CL> &sm, cg::cluster_group &cl, const TensorMeta &t, int mode) {
+    const int Q = t.dims[mode], LI = (t.dims[0] + 31) >> 5, NG = NW / LI;
+    static_assert(NW * 32 * RS <= MAXCHUNK * BMAXD * RS, "the groups' sums fit Mp");
+    for (int e = threadIdx.x; e < Q * (RS / 4); e += NW * 32) {
+        const int q = e / (RS / 4);
+        float4 v;
+        if (mode == 0) {
+            const float4 *p = reinterpret_cast<const float4 *>(&sm.Mp[0][0]);
+            v = p[e];
+            for (int g = 1; g < NG; g++) {
+                const float4 w = p[e + g * LI * 32 * (RS / 4)];
+                v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
             }
-            const double inv = 1.0 / piv;
-            for (int j = threadIdx.x; j < R; j += NT) {
-                sm.rowk[j] = (j == k ? 1.0 : sm.V[k + R * j]) * inv;
-                sm.colk[j] = sm.V[j + R * k];
-            }
-            __syncthreads();
-            for (int e = threadIdx.x; e < R * R; e += NT) {
-                const int i = e % R, j = e / R;
-                const double old = (j == k) ? 0.0 : sm.V[e];
-                sm.V[e] = (i == k) ? sm.rowk[j] : old - sm.colk[i] * sm.rowk[j];
-            }
-            __syncthreads();
+        } else {
+            int c = 0;  // rows Q c / CL .. are CTA c's
+            while (q >= Q * (c + 1) / CL) c++;
+            v = reinterpret_cast<const float4 *>(cl.map_shared_rank(sm.M, c))[e];
         }
-        __syncthreads();
-        if (!sm.fail) return;
-        if (threadIdx.x == 0 && attempt == 0) atomicAdd(a.fallbacks, 1);
-        __syncthreads();
+        reinterpret_cast<float4 *>(sm.Mg)[e] = v;
     }
 }
 
-// One ALS sweep of every tensor not yet converged: CTAs of NW warps pull
-// tensors from the queue.
-// Resident CTAs per SM the launch bounds ask for, per CTA width: 20, 18, 16
-// and 24 warps per SM (shared memory, ~45 KB a CTA, allows each); the
-// autotuner picks among the widths.
-constexpr int min_ctas(int nw) { return nw == 4 ? 5 : nw == 6 ? 3 : nw == 8 ? 2 : 2; }
-
-// (A register cap per width through __maxnreg__, 112 for six warps, cut
-// the spills but measured 2-7 % slower on the 4096-tensor batch.)
-template <int NW>
-__global__ void __launch_bounds__(NW * 32, min_ctas(NW)) k_batch_sweep(BatchArgs a) {
-    constexpr int NT = NW * 32;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    BatchSmem<NW> &sm = *reinterpret_cast<BatchSmem<NW> *>(smem_raw);
-    for (;;) {
-        if (threadIdx.x == 0) {
-            unsigned w = atomicAdd(a.queue, 1u);
-            sm.tensor = (w < (unsigned)a.ntensors) ? a.order[w] : -1;
+// sm.V = the inverse of the Hadamard of the Grams other than `mode`
+// (Gauss-Jordan, FP64): a cell per thread in registers, the pivot's row and
+// column published to double-buffered shared memory, one barrier a pivot; the
+// next pivot's owner takes its reciprocal.  Rows and columns past R are zero.
+// True when both attempts met a non-positive pivot (V is then not an inverse
+// and the caller keeps the old factor).
+template <int NW, int CL>
+__device__ bool normal_inverse_small(BatchSmem<NW, CL> &sm, int R, int mode, int *fallbacks) {
+    constexpr int NT = NW * 32, EP = (BMAXR * BMAXR + NT - 1) / NT;
+    for (int attempt = 0; attempt < 2; attempt++) {
+        double v[EP];
+        if (threadIdx.x < R) {
+            double d = 1.0;
+            for (int m = 0; m < 3; m++)
+                if (m != mode) d *= sm.G[m][threadIdx.x * (R + 1)];
+            sm.diag[threadIdx.x] = d;
         }
         __syncthreads();
-        const int ti = sm.tensor;
+        double maxdiag = 0.0;
+        for (int j = 0; j < R; j++) maxdiag = fmax(maxdiag, fabs(sm.diag[j]));
+        auto publish = [&](int k) {  // row, column and reciprocal of pivot k
+#pragma unroll
+            for (int q = 0; q < EP; q++) {
+                const int e = threadIdx.x + NT * q, i = e & (BMAXR - 1), j = e >> 4;
+                if (EP * NT > BMAXR * BMAXR && e >= BMAXR * BMAXR) continue;
+                if (i == k) sm.row[k & 1][j] = v[q];
+                if (j == k) sm.col[k & 1][i] = v[q];
+                if (i == k && j == k) sm.inv[k & 1] = 1.0 / v[q];
+            }
+        };
+#pragma unroll
+        for (int q = 0; q < EP; q++) {
+            const int e = threadIdx.x + NT * q, i = e & (BMAXR - 1), j = e >> 4;
+            v[q] = 0.0;
+            if (i < R && j < R) {
+                double x = 1.0;
+                for (int m = 0; m < 3; m++)
+                    if (m != mode) x *= sm.G[m][i + R * j];
+                if (attempt == 1 && i == j) x += 1e-10 * maxdiag + 1e-300;
+                v[q] = x;
+            }
+        }
+        bool fail = false;
+        publish(0);
+        for (int k = 0; k < R; k++) {
+            __syncthreads();
+            const double *row = sm.row[k & 1], *col = sm.col[k & 1];
+            const double piv = row[k], inv = sm.inv[k & 1];
+            if (!(piv > 1e-14 * maxdiag) || !isfinite(piv)) {
+                fail = true;  // the same on every thread
+                break;
+            }
+#pragma unroll
+            for (int q = 0; q < EP; q++) {
+                const int e = threadIdx.x + NT * q, i = e & (BMAXR - 1), j = e >> 4;
+                if (EP * NT > BMAXR * BMAXR && e >= BMAXR * BMAXR) continue;
+                const double rk = (j == k ? 1.0 : row[j]) * inv;
+                const double old = (j == k) ? 0.0 : v[q];
+                v[q] = (i == k) ? rk : old - col[i] * rk;
+            }
+            if (k + 1 < R) publish(k + 1);
+        }
+        if (!fail) {
+#pragma unroll
+            for (int q = 0; q < EP; q++) {
+                const int e = threadIdx.x + NT * q, i = e & (BMAXR - 1), j = e >> 4;
+                if (EP * NT > BMAXR * BMAXR && e >= BMAXR * BMAXR) continue;
+                sm.V[i * RS + j] = v[q];
+            }
+            __syncthreads();
+            return false;
+        }
         __syncthreads();
+        if (threadIdx.x == 0 && attempt == 0 && fallbacks) atomicAdd(fallbacks, 1);
+    }
+    return true;
+}
+
+// Sum over the CTA in a fixed order, the same on every thread; `red` holds a
+// slot per warp.
+template <int NW>
+__device__ double block_sum(double v, double *red) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+    for (int w = 0; w < NW; w++) v += red[w];
+    return v;
+}
+
+// One ALS sweep of every tensor not yet converged: clusters of CL CTAs of NW
+// warps pull tensors from the queue.  The CTAs of a cluster share a tensor's
+// MTTKRPs (outer index ranges), gather the result through distributed shared
+// memory and then run the R x R side and the factor update redundantly, so
+// each holds all factors.  The update U = M V^-1 and the Gram U^T U run on
+// the FP64 matrix instruction.
+// Six warps a CTA: one, two or three 32-row chunks divide them, so none idles.
+template <int NW, int CL>
+__global__ void __launch_bounds__(NW * 32, 2) k_batch_sweep(BatchArgs a) {
+    constexpr int NT = NW * 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BatchSmem<NW, CL> &sm = *reinterpret_cast<BatchSmem<NW, CL> *>(smem_raw);
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = CL > 1 ? (int)cl.block_rank() : 0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t mails = 0;  // mails that this warp has waited for
+    if (CL > 1 && threadIdx.x < NW) {
+        ptx::mbar_init(&sm.mail_full[threadIdx.x], 1);
+        ptx::fence_mbar_init();  // (the cluster synchronises before the first mail)
+    }
+    for (;;) {
+        if (rank == 0 && threadIdx.x == 0) {
+            const unsigned w = atomicAdd(a.queue, 1u);
+            const int ti = (w < (unsigned)a.ntensors) ? a.order[w] : -1;
+            if (CL > 1) {
+                for (int c = 0; c < CL; c++) *cl.map_shared_rank(&sm.tensor, c) = ti;
+            } else {
+                sm.tensor = ti;
+            }
+        }
+        if (CL > 1) cl.sync();
+        else __syncthreads();
+        const int ti = sm.tensor;
+        if (CL > 1) cl.sync();  // everyone has read it (and is still there) before it is written again
+        else __syncthreads();
         if (ti < 0) return;
         TensorMeta &t = a.meta[ti];
         if (t.done) continue;
@@ -345,51 +553,84 @@ __global__ void __launch_bounds__(NW * 32, min_ctas(NW)) k_batch_sweep(BatchArgs
         __syncthreads();
         double inner = 0.0;
         for (int mode = 0; mode < 3; mode++) {
-            if (R <= 4) mttkrp_lanes<NW, 4>(sm, a, t, mode);
-            else if (R <= 8) mttkrp_lanes<NW, 8>(sm, a, t, mode);
-            else mttkrp_lanes<NW, 16>(sm, a, t, mode);
-            normal_inverse_small<NT>(sm, a, t, mode);
-            // U_mode = M V^-1 (FP64 accumulation), into shared (row-major)
-            // and global (column-major) memory
+            if (R <= 4) mttkrp_lanes<4, NW, CL>(sm, cl, a, t, mode, rank, mails);
+            else if (R <= 8) mttkrp_lanes<8, NW, CL>(sm, cl, a, t, mode, rank, mails);
+            else mttkrp_lanes<16, NW, CL>(sm, cl, a, t, mode, rank, mails);
+            const float *M = sm.M;
+            if (CL > 1) {
+                cl.sync();  // every CTA's M is written
+                gather(sm, cl, t, mode);
+                M = sm.Mg;
+                cl.sync();  // and read, before the next mode's
+            }
+            const bool keep = normal_inverse_small(sm, R, mode, rank == 0 ? a.fallbacks : nullptr);
+            // U = M V^-1, 8 rows a warp at a time, into shared (row-major)
+            // and, a CTA's share of the rows, global (column-major) memory;
+            // singular twice: the old factor is kept
             const int Q = t.dims[mode];
-            float *Ug = a.U + t.uoff[mode];
-            const bool keep = sm.fail != 0;  // singular twice: keep the old factor
+            float *Ug = a.U + t.uoff[mode], *F = sm.F[mode];
             double part = 0.0;
-            for (int e = threadIdx.x; e < Q * R; e += NT) {
-                const int q = e % Q, c = e / Q;
-                float u = sm.F[mode][q * RS + c];
+            for (int q0 = 8 * warp; q0 < Q; q0 += 8 * NW) {
+                const int q = q0 + (lane >> 2);
+                double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
                 if (!keep) {
-                    double s = 0.0;
-                    for (int r = 0; r < R; r++) s = fma((double)sm.M[q * RS + r], sm.V[r + R * c], s);
-                    u = (float)s;
-                    sm.F[mode][q * RS + c] = u;
-                    Ug[e] = u;
+#pragma unroll
+                    for (int k = 0; k < BMAXR; k += 4) {
+                        const int r = k + (lane & 3);
+                        const double m = (q < Q && r < R) ? (double)M[q * RS + r] : 0.0;
+#pragma unroll
+                        for (int h = 0; h < 2; h++) dmma(c[h], m, sm.V[r * RS + 8 * h + (lane >> 2)]);
+                    }
                 }
-                if (mode == 2) part += (double)sm.M[q * RS + c] * (double)u;
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const int col = 8 * h + 2 * (lane & 3) + j;
+                        if (q >= Q || col >= R) continue;
+                        float u = F[q * RS + col];
+                        if (!keep) {
+                            u = (float)c[h][j];
+                            F[q * RS + col] = u;
+                            if (CL == 1 || (q0 >> 3) % CL == rank) Ug[q + Q * col] = u;
+                        }
+                        if (mode == 2) part += (double)M[q * RS + col] * (double)u;
+                    }
             }
             __syncthreads();
-            // Gram of the new factor
-            for (int e = threadIdx.x; e < R * R; e += NT) {
-                const int p = e % R, q2 = e / R;
-                double s = 0.0;
-                for (int i = 0; i < Q; i++) s = fma((double)sm.F[mode][i * RS + p], (double)sm.F[mode][i * RS + q2], s);
-                t.G[mode][e] = s;
+            // Gram of the new factor: a warp per 8 x 8 tile, the rows in
+            // order (as one chain of fused multiply-adds)
+            for (int tile = warp; tile < 4; tile += NW) {
+                const int p0 = 8 * (tile & 1), q0 = 8 * (tile >> 1);
+                double c[2] = {0.0, 0.0};
+#pragma unroll 4
+                for (int i0 = 0; i0 < Q; i0 += 4) {
+                    const int i = i0 + (lane & 3);
+                    const double f = i < Q ? (double)F[i * RS + p0 + (lane >> 2)] : 0.0;
+                    const double h = i < Q ? (double)F[i * RS + q0 + (lane >> 2)] : 0.0;
+                    dmma(c, f, h);
+                }
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const int p = p0 + (lane >> 2), q = q0 + 2 * (lane & 3) + j;
+                    if (p < R && q < R) sm.G[mode][p + R * q] = c[j];
+                }
             }
-            if (mode == 2) {
-                for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-                if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = part;
-            }
+            if (mode == 2) inner = block_sum<NW>(part, sm.red);
             __syncthreads();
-            if (mode == 2 && threadIdx.x == 0) {
-                for (int w = 0; w < NW; w++) inner += sm.red[w];
-            }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double hat = 0.0;
-            for (int e = 0; e < R * R; e++) hat += t.G[0][e] * t.G[1][e] * t.G[2][e];
-            const double res2 = t.normx2 - 2.0 * inner + hat;
-            const double fit = 1.0 - sqrt(res2 > 0.0 ? res2 : 0.0) / sqrt(t.normx2);
+        double hat = 0.0;
+        for (int e = threadIdx.x; e < R * R; e += NT) hat += sm.G[0][e] * sm.G[1][e] * sm.G[2][e];
+        hat = block_sum<NW>(hat, sm.red + NW);
+        if (rank == 0) {
+            for (int m = 0; m < 3; m++)
+                for (int e = threadIdx.x; e < R * R; e += NT) t.G[m][e] = sm.G[m][e];
+        }
+        if (rank == 0 && threadIdx.x == 0) {
+            double normx2 = 0.0;
+            for (int k = 0; k < NORM_PARTS; k++) normx2 += t.normp[k];
+            const double res2 = normx2 - 2.0 * inner + hat;
+            const double fit = 1.0 - sqrt(res2 > 0.0 ? res2 : 0.0) / sqrt(normx2);
             t.fit_prev = t.fit;
             t.fit = fit;
             t.sweeps += 1;
@@ -403,25 +644,28 @@ __global__ void __launch_bounds__(NW * 32, min_ctas(NW)) k_batch_sweep(BatchArgs
     }
 }
 
-// Per-tensor ||X||^2 and the initial Grams.
+// Per-tensor ||X||^2 (NORM_PARTS CTAs a tensor, a part of X each) and the
+// initial Grams (the first of them).
 __global__ void __launch_bounds__(256) k_batch_setup(TensorMeta *meta, int ntensors, const float *X,
                                                      const float *U) {
     __shared__ double red[8];
-    for (int ti = blockIdx.x; ti < ntensors; ti += gridDim.x) {
+    for (int b = blockIdx.x; b < ntensors * NORM_PARTS; b += gridDim.x) {
+        const int ti = b / NORM_PARTS, part = b % NORM_PARTS;
         TensorMeta &t = meta[ti];
-        const long n = (long)t.dims[0] * t.dims[1] * t.dims[2];
-        double s = 0.0;
-        for (long e = threadIdx.x; e < n; e += 256) {
-            const double x = X[t.xoff + e];
-            s += x * x;
+        const int n = t.dims[0] * t.dims[1] * t.dims[2];
+        const int e1 = (int)((long)n * (part + 1) / NORM_PARTS);
+        const float *x = X + t.xoff;
+        double s0 = 0.0;
+#pragma unroll 8
+        for (int e = (int)((long)n * part / NORM_PARTS) + threadIdx.x; e < e1; e += 256) {
+            const double v = __ldg(x + e);
+            s0 = fma(v, v, s0);
         }
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+        const double tot = block_sum<8>(s0, red);
+        if (threadIdx.x == 0) t.normp[part] = tot;
         __syncthreads();
+        if (part) continue;
         if (threadIdx.x == 0) {
-            double tot = 0.0;
-            for (int w = 0; w < 8; w++) tot += red[w];
-            t.normx2 = tot;
             t.fit = 0.0;
             t.fit_prev = 0.0;
             t.sweeps = 0;
@@ -434,11 +678,11 @@ __global__ void __launch_bounds__(256) k_batch_setup(TensorMeta *meta, int ntens
             for (int e = threadIdx.x; e < R * R; e += 256) {
                 const int p = e % R, q = e / R;
                 double g = 0.0;
+#pragma unroll 8
                 for (int i = 0; i < I; i++) g = fma((double)F[i + I * p], (double)F[i + I * q], g);
                 t.G[m][e] = g;
             }
         }
-        __syncthreads();
     }
 }
 
@@ -449,38 +693,64 @@ struct BatchState {
     int *fallbacks = nullptr;
 };
 
-template <int NW>
+template <int NW, int CL>
 int launch_sweep(const BatchArgs &a, int ctas_per_sm, cudaStream_t s) {
     static std::atomic<bool> attr[64];  // per device; zero-initialised
+    using Smem = BatchSmem<NW, CL>;
     int dev = 0;
     CUD_CHECK(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !attr[dev].load(std::memory_order_acquire)) {
-        CUD_CHECK(cudaFuncSetAttribute(k_batch_sweep<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(BatchSmem<NW>)));
+    if (dev < 0 || dev >= 64 || !attr[dev].load(std::memory_order_acquire)) {
+        CUD_CHECK(cudaFuncSetAttribute(k_batch_sweep<NW, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(Smem)));
         // the whole unified L1 as shared memory: the CTAs per SM the tuner
         // asks for are then limited by shared memory, not by the carveout
-        CUD_CHECK(cudaFuncSetAttribute(k_batch_sweep<NW>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        CUD_CHECK(cudaFuncSetAttribute(k_batch_sweep<NW, CL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
-        attr[dev].store(true, std::memory_order_release);
+        if (dev >= 0 && dev < 64) attr[dev].store(true, std::memory_order_release);
     }
     CUD_CHECK(cudaMemsetAsync(a.queue, 0, sizeof(unsigned), s));
-    k_batch_sweep<NW><<<kNumSMs * ctas_per_sm, NW * 32, sizeof(BatchSmem<NW>), s>>>(a);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CL;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    // no more clusters than tensors
+    cfg.gridDim = dim3((unsigned)(std::min((long)kNumSMs * ctas_per_sm / CL, (long)a.ntensors) * CL));
+    cfg.blockDim = dim3(NW * 32);
+    cfg.dynamicSmemBytes = sizeof(Smem);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = CL > 1 ? 1 : 0;
+    CUD_CHECK(cudaLaunchKernelEx(&cfg, k_batch_sweep<NW, CL>, a));
     CUD_CHECK_LAUNCH("batched sweep");
     return CUD_OK;
 }
 
-// Launch shape: threads per CTA (warps x 32) and CTAs per SM.
+// Launch shape: threads per CTA (warps x 32), CTAs per SM, CTAs per tensor.
 struct BatchCfg {
-    int threads, ctas;
+    int threads, ctas, cluster;
 };
 
 int launch_cfg(const BatchArgs &a, const BatchCfg &c, cudaStream_t s) {
-    switch (c.threads) {
-        case 128: return launch_sweep<4>(a, c.ctas, s);
-        case 192: return launch_sweep<6>(a, c.ctas, s);
-        case 256: return launch_sweep<8>(a, c.ctas, s);
-        default: return launch_sweep<12>(a, c.ctas, s);
-    }
+    if (c.cluster == 8) return launch_sweep<6, 8>(a, c.ctas, s);
+    if (c.cluster == 4) return launch_sweep<6, 4>(a, c.ctas, s);
+    if (c.cluster == 2) return launch_sweep<6, 2>(a, c.ctas, s);
+    return launch_sweep<6, 1>(a, c.ctas, s);
+}
+
+// The launch shape of a batch that was not tuned: as many CTAs a tensor as
+// the SMs are short of tensors (a CTA alone takes most of a millisecond for a
+// sweep of the largest).  B200, ms a sweep with setup, dims 16 to 96, ranks 4
+// to 16, clusters of 1 / 2 / 4 / 8: 64 tensors 0.52 / 0.31 / 0.24 / 0.23;
+// 148: 0.51 / 0.41 / 0.31 / 0.45; 256: 0.87 / 0.49 / 0.48 / 0.72; 512: 1.13 /
+// 0.86 / 1.06 / 1.55; 1024: 1.59 / 1.63 / 2.00 / -; 2048: 2.90 / 3.19 / 3.93.
+// (Six warps a CTA of 2 x 8 register tiles without clusters: 0.92 ms at 64,
+// 1.28 at 256, 2.0 at 1024, 3.2 at 2048.)
+BatchCfg default_cfg(int n) {
+    if (n <= kNumSMs / 2) return {192, 2, 8};
+    if (n <= 2 * kNumSMs) return {192, 2, 4};
+    if (n <= 6 * kNumSMs) return {192, 2, 2};
+    return {192, 2, 1};
 }
 
 // Autotuner cache: shape class -> launch shape
@@ -551,6 +821,7 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
     a.queue = reinterpret_cast<unsigned *>(w + sizeof(TensorMeta) * ntensors + sizeof(int) * ntensors);
     a.fallbacks = reinterpret_cast<int *>(a.queue + 16);
     a.ndone = reinterpret_cast<int *>(a.queue + 32);
+    a.error = a.ndone + 1;
     a.ntensors = ntensors;
     a.X = X;
     a.U = U;
@@ -560,12 +831,12 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
     CUD_CHECK(cudaMemcpyAsync(const_cast<int *>(a.order), order.data(), sizeof(int) * ntensors,
                               cudaMemcpyHostToDevice, s));
     CUD_CHECK(cudaMemsetAsync(a.queue, 0, 256, s));
-    k_batch_setup<<<std::min(ntensors, kNumSMs * 4), 256, 0, s>>>(a.meta, ntensors, X, U);
+    k_batch_setup<<<std::min((long)ntensors * NORM_PARTS, kNumSMs * 64L), 256, 0, s>>>(a.meta, ntensors, X, U);
     CUD_CHECK_LAUNCH("batched setup");
 
     // launch shape from the autotuner (threads per CTA, CTAs per SM, tile rows)
     long key = shape_class(ntensors, hd.data(), hr.data());
-    BatchCfg cfg{192, 3};
+    BatchCfg cfg = default_cfg(ntensors);
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune.find(key);
@@ -604,10 +875,11 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
         }
         launched += per;
         done_sweeps += per;
-        // convergence check: the count of converged tensors (4 bytes)
-        if (!ndone_h || cudaMemcpyAsync(ndone_h, a.ndone, sizeof(int), cudaMemcpyDeviceToHost, cs) != cudaSuccess ||
+        // convergence check: the count of converged tensors, and the error flag
+        if (!ndone_h || cudaMemcpyAsync(ndone_h, a.ndone, 2 * sizeof(int), cudaMemcpyDeviceToHost, cs) != cudaSuccess ||
             cudaStreamSynchronize(cs) != cudaSuccess) { st = CUD_ERR_CUDA; break; }
-        if (*ndone_h >= ntensors) break;
+        if (ndone_h[1]) { st = CUD_ERR_DEVICE_TIMEOUT; break; }
+        if (ndone_h[0] >= ntensors) break;
     }
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -662,8 +934,8 @@ extern "C" int cud_cp_batched_tune(int ntensors, const long *dims, const long *r
     long key = shape_class(ntensors, hd.data(), hr.data());
     // (threads, CTAs per SM) within the launch bounds' register budgets and
     // shared memory (~45 KB a CTA)
-    const std::vector<BatchCfg> cand = {{128, 4}, {128, 5}, {192, 3}, {256, 2}, {384, 2}};
-    BatchCfg bestc{192, 3};
+    const std::vector<BatchCfg> cand = {{192, 2, 1}, {192, 2, 2}, {192, 2, 4}, {192, 2, 8}};
+    BatchCfg bestc = default_cfg(ntensors);
     cudaStream_t s = as_stream(stream);
     cudaEvent_t e0, e1;
     CUD_CHECK(cudaEventCreate(&e0));

@@ -291,5 +291,37 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ---------------------------------------------------------------- clusters
+
+__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
+
+// Arrives on the barrier at the same shared-memory offset of CTA `cta` of the
+// cluster, releasing this thread's writes (also to that CTA's shared memory).
+__device__ __forceinline__ void mbar_arrive_cluster(uint64_t *bar, int cta) {
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(smem_addr(bar)),
+        "r"(cta)
+        : "memory");
+}
+
+// Waits (bounded: false when it ran out) for a phase of this CTA's barrier
+// that threads of the cluster complete, acquiring their writes.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity) {
+    for (int it = 0; it < 20000; it++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_addr(bar)), "r"(parity), "r"(100000u)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
 }  // namespace ptx
 }  // namespace cud
