@@ -53,14 +53,19 @@ struct TensorMeta {
     int R;
     int done;
     int sweeps;
-    double normp[NORM_PARTS];  // ||X||^2 by parts of the tensor
     double fit, fit_prev;
     double target;      // stop once fit >= target (<= 0: no target)
+};
+
+// What a tensor keeps on the device alone between sweeps.
+struct TensorState {
+    double normp[NORM_PARTS];    // ||X||^2 by parts of the tensor
     double G[3][BMAXR * BMAXR];  // factor Grams (FP64)
 };
 
 struct BatchArgs {
     TensorMeta *meta;
+    TensorState *state;
     const int *order;   // processing order (largest first)
     int ntensors;
     const float *X;
@@ -104,7 +109,7 @@ struct BatchSmem {
 static_assert(2 * (sizeof(BatchSmem<6, 8>) + 1024) <= 228 * 1024, "two CTAs an SM");
 
 template <int NT, class Smem>
-__device__ void load_factors(Smem &sm, const BatchArgs &a, const TensorMeta &t) {
+__device__ void load_factors(Smem &sm, const BatchArgs &a, const TensorMeta &t, const TensorState &g) {
     for (int m = 0; m < 3; m++) {
         const float *src = a.U + t.uoff[m];
         const int I = t.dims[m];
@@ -112,7 +117,7 @@ __device__ void load_factors(Smem &sm, const BatchArgs &a, const TensorMeta &t) 
             const int i = e / RS, r = e - i * RS;
             sm.F[m][e] = (r < t.R && i < I) ? src[i + I * r] : 0.f;
         }
-        for (int e = threadIdx.x; e < t.R * t.R; e += NT) sm.G[m][e] = t.G[m][e];
+        for (int e = threadIdx.x; e < t.R * t.R; e += NT) sm.G[m][e] = g.G[m][e];
     }
 }
 
@@ -549,7 +554,8 @@ __global__ void __launch_bounds__(NW * 32, 2) k_batch_sweep(BatchArgs a) {
         TensorMeta &t = a.meta[ti];
         if (t.done) continue;
         const int R = t.R;
-        load_factors<NT>(sm, a, t);
+        TensorState &ts = a.state[ti];
+        load_factors<NT>(sm, a, t, ts);
         __syncthreads();
         double inner = 0.0;
         for (int mode = 0; mode < 3; mode++) {
@@ -624,11 +630,11 @@ __global__ void __launch_bounds__(NW * 32, 2) k_batch_sweep(BatchArgs a) {
         hat = block_sum<NW>(hat, sm.red + NW);
         if (rank == 0) {
             for (int m = 0; m < 3; m++)
-                for (int e = threadIdx.x; e < R * R; e += NT) t.G[m][e] = sm.G[m][e];
+                for (int e = threadIdx.x; e < R * R; e += NT) ts.G[m][e] = sm.G[m][e];
         }
         if (rank == 0 && threadIdx.x == 0) {
             double normx2 = 0.0;
-            for (int k = 0; k < NORM_PARTS; k++) normx2 += t.normp[k];
+            for (int k = 0; k < NORM_PARTS; k++) normx2 += ts.normp[k];
             const double res2 = normx2 - 2.0 * inner + hat;
             const double fit = 1.0 - sqrt(res2 > 0.0 ? res2 : 0.0) / sqrt(normx2);
             t.fit_prev = t.fit;
@@ -646,12 +652,13 @@ __global__ void __launch_bounds__(NW * 32, 2) k_batch_sweep(BatchArgs a) {
 
 // Per-tensor ||X||^2 (NORM_PARTS CTAs a tensor, a part of X each) and the
 // initial Grams (the first of them).
-__global__ void __launch_bounds__(256) k_batch_setup(TensorMeta *meta, int ntensors, const float *X,
-                                                     const float *U) {
+__global__ void __launch_bounds__(256) k_batch_setup(TensorMeta *meta, TensorState *state, int ntensors,
+                                                     const float *X, const float *U) {
     __shared__ double red[8];
     for (int b = blockIdx.x; b < ntensors * NORM_PARTS; b += gridDim.x) {
         const int ti = b / NORM_PARTS, part = b % NORM_PARTS;
         TensorMeta &t = meta[ti];
+        TensorState &ts = state[ti];
         const int n = t.dims[0] * t.dims[1] * t.dims[2];
         const int e1 = (int)((long)n * (part + 1) / NORM_PARTS);
         const float *x = X + t.xoff;
@@ -662,7 +669,7 @@ __global__ void __launch_bounds__(256) k_batch_setup(TensorMeta *meta, int ntens
             s0 = fma(v, v, s0);
         }
         const double tot = block_sum<8>(s0, red);
-        if (threadIdx.x == 0) t.normp[part] = tot;
+        if (threadIdx.x == 0) ts.normp[part] = tot;
         __syncthreads();
         if (part) continue;
         if (threadIdx.x == 0) {
@@ -680,7 +687,7 @@ __global__ void __launch_bounds__(256) k_batch_setup(TensorMeta *meta, int ntens
                 double g = 0.0;
 #pragma unroll 8
                 for (int i = 0; i < I; i++) g = fma((double)F[i + I * p], (double)F[i + I * q], g);
-                t.G[m][e] = g;
+                ts.G[m][e] = g;
             }
         }
     }
@@ -788,7 +795,12 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
     if (opt_in) opt = *opt_in;
     if (opt.max_sweeps < 1) return set_status(CUD_ERR_INVALID_ARGUMENT);
     cudaStream_t s = as_stream(stream);
-    std::vector<TensorMeta> hm(ntensors);
+    // the tensors' descriptions and the processing order, uploaded as one
+    // block: [meta][order]; the device's own state follows it in the scratch
+    const size_t mbytes = (sizeof(TensorMeta) * ntensors + sizeof(int) * ntensors + 255) & ~size_t(255);
+    std::vector<double> host((mbytes + 7) / 8);
+    TensorMeta *hm = reinterpret_cast<TensorMeta *>(host.data());
+    int *order = reinterpret_cast<int *>(hm + ntensors);
     std::vector<int> hd(3 * ntensors), hr(ntensors);
     std::vector<std::pair<double, int>> work(ntensors);
     for (int t = 0; t < ntensors; t++) {
@@ -808,30 +820,27 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
         work[t] = {-(double)m.dims[0] * m.dims[1] * m.dims[2] * m.R, t};
     }
     std::sort(work.begin(), work.end());
-    std::vector<int> order(ntensors);
     for (int t = 0; t < ntensors; t++) order[t] = work[t].second;
 
     int st;
-    size_t bytes = sizeof(TensorMeta) * ntensors + sizeof(int) * ntensors + 256;
-    char *w = (char *)scratch(kSlotTmp1, bytes, &st);
+    char *w = (char *)scratch(kSlotTmp1, mbytes + 256 + sizeof(TensorState) * ntensors, &st);
     if (!w) return set_status(st);
     BatchArgs a;
     a.meta = reinterpret_cast<TensorMeta *>(w);
-    a.order = reinterpret_cast<int *>(w + sizeof(TensorMeta) * ntensors);
-    a.queue = reinterpret_cast<unsigned *>(w + sizeof(TensorMeta) * ntensors + sizeof(int) * ntensors);
+    a.order = reinterpret_cast<int *>(a.meta + ntensors);
+    a.queue = reinterpret_cast<unsigned *>(w + mbytes);
     a.fallbacks = reinterpret_cast<int *>(a.queue + 16);
     a.ndone = reinterpret_cast<int *>(a.queue + 32);
     a.error = a.ndone + 1;
+    a.state = reinterpret_cast<TensorState *>(w + mbytes + 256);
     a.ntensors = ntensors;
     a.X = X;
     a.U = U;
     a.max_sweeps = opt.max_sweeps;
     a.tol = opt.tol;
-    CUD_CHECK(cudaMemcpyAsync(a.meta, hm.data(), sizeof(TensorMeta) * ntensors, cudaMemcpyHostToDevice, s));
-    CUD_CHECK(cudaMemcpyAsync(const_cast<int *>(a.order), order.data(), sizeof(int) * ntensors,
-                              cudaMemcpyHostToDevice, s));
+    CUD_CHECK(cudaMemcpyAsync(w, hm, mbytes, cudaMemcpyHostToDevice, s));
     CUD_CHECK(cudaMemsetAsync(a.queue, 0, 256, s));
-    k_batch_setup<<<std::min((long)ntensors * NORM_PARTS, kNumSMs * 64L), 256, 0, s>>>(a.meta, ntensors, X, U);
+    k_batch_setup<<<std::min((long)ntensors * NORM_PARTS, kNumSMs * 64L), 256, 0, s>>>(a.meta, a.state, ntensors, X, U);
     CUD_CHECK_LAUNCH("batched setup");
 
     // launch shape from the autotuner (threads per CTA, CTAs per SM, tile rows)
@@ -844,9 +853,12 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
     }
     // sweeps: graph of `per` sweeps replayed; the done-count read back between
     const int per = std::max(1, std::min(opt.check_every > 1 ? opt.check_every : 5, opt.max_sweeps));
+    // a graph that would be replayed once is not built (capture, instantiation
+    // and a stream of its own took 0.4 ms of a call)
+    const bool use_graph = opt.use_graph && opt.max_sweeps > per;
     cudaStream_t cs = s;
     bool own = false;
-    if (s == nullptr || s == cudaStreamLegacy || s == cudaStreamPerThread) {
+    if (use_graph && (s == nullptr || s == cudaStreamLegacy || s == cudaStreamPerThread)) {
         CUD_CHECK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         own = true;
         CUD_CHECK(cudaStreamSynchronize(s));
@@ -854,7 +866,7 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     st = CUD_OK;
-    if (opt.use_graph) {
+    if (use_graph) {
         if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess) st = CUD_ERR_CUDA;
         for (int i = 0; i < per && st == CUD_OK; i++) st = launch_cfg(a, cfg, cs);
         cudaError_t e = cudaStreamEndCapture(cs, &graph);
