@@ -21,6 +21,7 @@
 // is close to 1 and inherits the MTTKRP's rounding), this value depends only
 // on X and the factors.
 #include "kernels.cuh"
+#include "tc_ptx.cuh"
 
 namespace cud {
 
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(NT) k_cp_residual(ResArgs a) {
 __global__ void __launch_bounds__(256) k_sum_pairs(const double *part, long n, double *out) {
     __shared__ double red[2][256];
     double s0 = 0.0, s1 = 0.0;
+    ptx::griddep_wait();  // the partials (launched programmatically behind the tensor-core residual)
     for (long b = threadIdx.x; b < n; b += 256) { s0 += part[2 * b]; s1 += part[2 * b + 1]; }
     red[0][threadIdx.x] = s0;
     red[1][threadIdx.x] = s1;
@@ -184,7 +186,8 @@ __global__ void __launch_bounds__(256) k_sum_pairs(const double *part, long n, d
 }  // namespace
 
 int sum_pairs(const double *part, long n, double *out, cudaStream_t s) {
-    k_sum_pairs<<<1, 256, 0, s>>>(part, n, out);
+    PdlLaunch l(1, 256, 0, s);
+    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, k_sum_pairs, part, n, out));
     CUD_CHECK_LAUNCH("cp_residual sum");
     return CUD_OK;
 }
@@ -451,12 +454,12 @@ int cp_residual_host(const float *X, int order, const long *dims, const float *c
     const size_t bytes = cp_residual_ws_bytes(order, dims);
     double *ws = static_cast<double *>(scratch(kSlotReduce, bytes, &st));
     if (!ws) return st;
-    double *out = ws + (bytes / sizeof(double) - 2);
-    st = cp_residual(X, order, dims, U, R, out, ws, s, need_x2);
-    if (st) return st;
+    // the last kernel writes its two sums to pinned host memory itself: no
+    // copy behind it
     double *h = pinned_scalars();
     if (!h) return CUD_ERR_NO_MEMORY;
-    CUD_CHECK(cudaMemcpyAsync(h, out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    st = cp_residual(X, order, dims, U, R, h, ws, s, need_x2);
+    if (st) return st;
     CUD_CHECK(cudaStreamSynchronize(s));
     if (res_norm2) *res_norm2 = h[0];
     if (x_norm2) *x_norm2 = h[1];

@@ -10,9 +10,9 @@
 // a 128-row tile of which is one MMA per 128 columns of U_1 with contraction
 // length R.  A CTA owns one 128-row tile of mode 0 and a contiguous range of
 // k; per k:
-//   * four builder warps form A' = U_0 rows times c_k (each thread holds its
-//     row of U_0 in registers), split it into BF16 hi and lo and store both
-//     in TMEM (double-buffered over k);
+//   * eight builder warps form A' = U_0 rows times c_k (each thread holds half
+//     of its row of U_0 in registers), split it into BF16 hi and lo and store
+//     both in TMEM (double-buffered over k);
 //   * one thread issues, per 128-column chunk of U_1, the three products
 //     A'_hi B_hi + A'_hi B_lo + A'_lo B_hi into a TMEM accumulator
 //     (double-buffered over chunks); B = U_1 split into hi and lo once per CTA
@@ -20,10 +20,17 @@
 //   * one thread streams the matching X tiles (128 rows x 32 columns,
 //     TMA, a ring as deep as the shared memory beside U_1 allows, 2-12
 //     tiles) -- X is read exactly once;
-//   * eight epilogue warps (two per TMEM lane quarter, each half of the
-//     columns) read the accumulator row by row (tcgen05.ld) and the X tile
-//     from shared memory and add (x - xh)^2 (per tile in FP32) and x^2 (in
-//     FP64) into FP64 totals, four independent sums each.
+//   * sixteen epilogue warps (four per TMEM lane quarter, one for each of a
+//     chunk's four X tiles) read the accumulator row by row (tcgen05.ld) and
+//     the X tile from shared memory and add (x - xh)^2 (16 columns at a time
+//     in FP32) and x^2 (in FP64) into FP64 totals, four independent sums each;
+//     tiles past I_1 are neither loaded nor read, rows past I_0 not read.
+// Bound: HBM (X once); what it runs into is the epilogue's chain per chunk
+// (barrier, TMEM and shared-memory loads, FP64 conversions at a quarter of a
+// warp a clock), hence the many warps.  B200: 512^3 R = 64 182 -> 131 us
+// (eight epilogue warps that each waited for every tile, and 64-bit divisions
+// for the ring positions), 384^3 87 -> 62, 96^4 R = 32 209 -> 129.
+// (CTAs that share U_1's chunks, with rings of 12 tiles, form A' oftener: 144.)
 // Rows past I_0 and columns past I_1 are zero in A' and B and in the X tiles
 // (the TMA fill), so they add nothing.  Per-CTA totals are summed in a fixed
 // order by k_sum_pairs (deterministic).  Every wait is bounded; a CTA that
@@ -52,8 +59,9 @@ constexpr int RT_XJ = 32;       // U_1 rows (X columns) per X tile
 // bound by its per-slice chain (A' build -> MMA -> epilogue), not by the
 // bytes in flight.
 constexpr int RT_XSMAX = 12;
-constexpr int RT_THREADS = 448; // warp 0 TMA, 1 MMA, 2-5 builders, 6-13 epilogue
-constexpr int RT_EPI = 8;       // epilogue warps: two per TMEM lane quarter, 16 of every 32 columns each
+constexpr int RT_THREADS = 832; // warp 0 TMA, 1 MMA, 2-9 builders, 10-25 epilogue
+constexpr int RT_BLD = 8;       // builder warps: two per TMEM lane quarter, 32 ranks each
+constexpr int RT_EPI = 16;      // epilogue warps: four per TMEM lane quarter, an X tile of a chunk each
 constexpr uint32_t RT_XBYTES = RT_ROWS * RT_XJ * 4;
 constexpr int RT_RMAX = 64;
 constexpr int RT_BMAX = 128 * 1024;  // U_1 hi + lo in shared memory
@@ -77,7 +85,7 @@ struct RtCtrl {
     int abort;
     const float *fU[kMaxOrder];
     long frows[kMaxOrder];
-    float cvec[4][RT_RMAX];
+    float cvec[RT_BLD][32];
     double red[2][RT_EPI];
 };
 constexpr size_t RT_CTRL_BYTES = (sizeof(RtCtrl) + 1023) & ~size_t(1023);
@@ -107,6 +115,24 @@ __device__ __forceinline__ void rt_split_pair(float a, float b, uint32_t &hi, ui
     lo = rt_pack_bf16(a - f.x, b - f.y);
 }
 
+// Position in the X ring, advanced by counters: a 64-bit division and a
+// remainder per tile were most of the epilogue's time (384^3 R64: 86 us a
+// launch).
+struct RtRing {
+    int slot = 0, n;
+    uint32_t use = 0;
+    __device__ explicit RtRing(int n_) : n(n_) {}
+    __device__ __forceinline__ void next() {
+        if (++slot == n) {
+            slot = 0;
+            use++;
+        }
+    }
+    __device__ __forceinline__ void next(int step) {
+        for (slot += step; slot >= n; slot -= n) use++;
+    }
+};
+
 __global__ void __launch_bounds__(RT_THREADS, 1)
     k_residual_tc(const __grid_constant__ CUtensorMap tmap, RtArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -126,10 +152,10 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
     if (threadIdx.x == 0) {
         for (int i = 0; i < RT_XSMAX; i++) {
             ptx::mbar_init(&sm.x_full[i], 1);
-            ptx::mbar_init(&sm.x_empty[i], RT_EPI);  // the epilogue warps
+            ptx::mbar_init(&sm.x_empty[i], 4);  // the tile's epilogue warps, one per lane quarter
         }
         for (int b = 0; b < 2; b++) {
-            ptx::mbar_init(&sm.a_full[b], 4);   // the builder warps
+            ptx::mbar_init(&sm.a_full[b], RT_BLD);   // the builder warps
             ptx::mbar_init(&sm.a_free[b], 1);   // tcgen05.commit
             ptx::mbar_init(&sm.d_full[b], 1);   // tcgen05.commit
             ptx::mbar_init(&sm.d_free[b], RT_EPI);   // the epilogue warps
@@ -144,6 +170,24 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
         ptx::fence_mbar_init();
         ptx::prefetch_tmap(&tmap);
     }
+    // X tile loads (thread 0): the first ring of them go out before B is built
+    RtRing xl(a.xs);
+    long xk = 0, issued_x = 0;
+    int xt = 0;
+    const int ntiles = (int)((a.I1 + RT_XJ - 1) / RT_XJ);  // X tiles per k
+    auto load_x = [&]() {
+        ptx::mbar_arrive_expect_tx(&sm.x_full[xl.slot], RT_XBYTES);
+        ptx::tma_load_3d(xring + (size_t)xl.slot * RT_XBYTES, &tmap, &sm.x_full[xl.slot], (int)i0,
+                         xt * RT_XJ, (int)(k_beg + xk));
+        issued_x++;
+        xl.next();
+        if (++xt == ntiles) {
+            xt = 0;
+            xk++;
+        }
+    };
+    if (threadIdx.x == 0)
+        while (xk < nk && xl.use == 0) load_x();
     if (warp == 0) {
         ptx::tmem_alloc(&sm.tmem_base, RT_TMEM_COLS);
         ptx::tmem_relinquish();
@@ -153,18 +197,18 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
     // form one 16-byte word at jr * 16 + kc * 2048 (descriptor: 8-row groups
     // 128 B apart, K chunks 2048 B apart)
     {
-        const int kcs = a.Rpad / 8;
-        const long items = (long)a.nq * RT_NJ * kcs;
-        for (long it = threadIdx.x; it < items; it += RT_THREADS) {
+        const unsigned kcs = (unsigned)a.Rpad / 8, items = (unsigned)a.nq * RT_NJ * kcs;
+#pragma unroll 2
+        for (unsigned it = threadIdx.x; it < items; it += RT_THREADS) {
             const int jr = (int)(it % RT_NJ);
-            const long rest = it / RT_NJ;
-            const int kc = (int)(rest % kcs), q = (int)(rest / kcs);
+            const unsigned rest = it / RT_NJ;
+            const int q = (int)(rest / kcs), kc = (int)(rest - q * kcs);
             const long j = (long)q * RT_NJ + jr;
             float v[8];
 #pragma unroll
             for (int e = 0; e < 8; e++) {
                 const int r = 8 * kc + e;
-                v[e] = (j < a.I1 && r < a.R) ? a.U1[j + a.I1 * r] : 0.f;
+                v[e] = (j < a.I1 && r < a.R) ? __ldg(a.U1 + j + a.I1 * r) : 0.f;
             }
             uint4 h, l;
             rt_split_pair(v[0], v[1], h.x, l.x);
@@ -184,24 +228,13 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;  // a warp's TMEM lane quarter
     const int row = (warp & 3) * 32 + lane;                       // tile row of builder / epilogue threads
 
-    long issued_x = 0;
     double s_res = 0.0, s_x = 0.0;
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
-            long xi = 0;
-            for (long kl = 0; kl < nk && !*abort; kl++) {
-                for (int q = 0; q < a.nq && !*abort; q++) {
-                    for (int s = 0; s < RT_NJ / RT_XJ; s++, xi++) {
-                        const int slot = (int)(xi % a.xs);
-                        const long use = xi / a.xs;
-                        if (use > 0 && !ptx::mbar_wait(&sm.x_empty[slot], (uint32_t)((use - 1) & 1), abort)) break;
-                        ptx::mbar_arrive_expect_tx(&sm.x_full[slot], RT_XBYTES);
-                        ptx::tma_load_3d(xring + (size_t)slot * RT_XBYTES, &tmap, &sm.x_full[slot], (int)i0,
-                                         q * RT_NJ + s * RT_XJ, (int)(k_beg + kl));
-                        issued_x = xi + 1;
-                    }
-                }
+            while (xk < nk && !*abort) {
+                if (!ptx::mbar_wait(&sm.x_empty[xl.slot], (uint32_t)((xl.use - 1) & 1), abort)) break;
+                load_x();
             }
         }
     } else if (warp == 1) {
@@ -239,41 +272,40 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
             for (long it = 0; it < 40000 && !ptx::mbar_try_wait_hint(&sm.done, 0, 100000u); it++) {
             }
         }
-    } else if (warp < 6) {
+    } else if (warp < 2 + RT_BLD) {
         // ------------------------------------------------------------ A' builders
         const long i = i0 + row;
-        float u0[RT_RMAX];
+        const int h = (warp - 2) >> 2;  // ranks 32 h ..
+        float u0[32];
 #pragma unroll
-        for (int r = 0; r < RT_RMAX; r++) u0[r] = (i < a.I0 && r < a.R) ? a.U0[i + a.I0 * r] : 0.f;
+        for (int r = 0; r < 32; r++) u0[r] = (i < a.I0 && 32 * h + r < a.R) ? __ldg(a.U0 + i + a.I0 * (32 * h + r)) : 0.f;
         float *cv = sm.cvec[warp - 2];
         for (long kl = 0; kl < nk && !*abort; kl++) {
             const int b = (int)(kl & 1);
-            // c_k for r = lane, lane + 32: the slower factors' rows of k
-            const long k = k_beg + kl;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int r = lane + 32 * h;
+            // c_k at this lane's rank: the slower factors' rows of k
+            {
+                const int r = 32 * h + lane;
                 float c = 0.f;
                 if (r < a.R) {
                     c = 1.f;
-                    long rem = k;
+                    uint32_t rem = (uint32_t)(k_beg + kl);  // K < 2^31
                     for (int f = 0; f < a.f.n; f++) {
-                        const long d = rem % sm.frows[f];
-                        rem /= sm.frows[f];
-                        c *= sm.fU[f][d + sm.frows[f] * r];
+                        const uint32_t rows = (uint32_t)sm.frows[f], q = rem / rows;
+                        c *= __ldg(sm.fU[f] + (rem - q * rows) + (long)rows * r);
+                        rem = q;
                     }
                 }
-                cv[r] = c;
+                cv[lane] = c;
             }
             __syncwarp();
             if (kl >= 2 && !*abort) ptx::mbar_wait(&sm.a_free[b], (uint32_t)(((kl >> 1) - 1) & 1), abort);
             const bool ok = __all_sync(0xffffffffu, *abort == 0);  // warp-uniform exit before tcgen05.st
             if (!ok) break;
             ptx::tc_fence_after();
-            const uint32_t a_hi = tbase + lane_off + 2u * RT_NJ + (uint32_t)b * 64u, a_lo = a_hi + 32u;
+            const uint32_t a_hi = tbase + lane_off + 2u * RT_NJ + (uint32_t)b * 64u + 16u * h, a_lo = a_hi + 32u;
 #pragma unroll
-            for (int g = 0; g < RT_RMAX / 16; g++) {
-                if (g < a.Rpad / 16) {
+            for (int g = 0; g < 2; g++) {
+                if (2 * h + g < a.Rpad / 16) {
                     uint32_t hi[8], lo[8];
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
@@ -291,52 +323,53 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
         }
     } else {
         // ------------------------------------------------------------ epilogue
-        const int hcol = ((warp - 6) >> 2) * (RT_XJ / 2);  // this warp's 16 columns of each tile
+        const int g = (warp - 2 - RT_BLD) >> 2;                // this warp's X tile of each chunk
+        const bool rows = i0 + (row & ~31) < a.I0;             // its 32 rows hold any of the tensor's
         double sr[4] = {0.0, 0.0, 0.0, 0.0}, sx[4] = {0.0, 0.0, 0.0, 0.0};
-        long ci = 0, xi = 0;
-        for (; ci < nchunks && !*abort; ci++) {
+        RtRing xr(a.xs);
+        xr.next(g);
+        int q = 0;
+        for (long ci = 0; ci < nchunks && !*abort; ci++) {
             const int db = (int)(ci & 1);
+            const int tiles = min(RT_NJ / RT_XJ, ntiles - q * (RT_NJ / RT_XJ));  // X tiles of the chunk
+            const bool mine = g < tiles;
             if (!*abort) ptx::mbar_wait(&sm.d_full[db], (uint32_t)((ci >> 1) & 1), abort);
+            if (mine && !*abort) ptx::mbar_wait(&sm.x_full[xr.slot], (uint32_t)(xr.use & 1), abort);
             const bool ok = __all_sync(0xffffffffu, *abort == 0);  // warp-uniform exit before tcgen05.ld
             if (!ok) break;
-            ptx::tc_fence_after();
-            // the chunk's accumulator columns of this warp, four loads and one wait
-            uint32_t v[RT_NJ / RT_XJ][16];
+            if (mine && rows) {
+                ptx::tc_fence_after();
+                const float *xs = reinterpret_cast<const float *>(xring + (size_t)xr.slot * RT_XBYTES) + row;
+                uint32_t v[2][16];
 #pragma unroll
-            for (int s = 0; s < RT_NJ / RT_XJ; s++)
-                ptx::tmem_ld16(tbase + lane_off + (uint32_t)db * RT_NJ + (uint32_t)(s * RT_XJ + hcol), v[s]);
-            ptx::tmem_wait_ld();
-            bool stop = false;
+                for (int h = 0; h < 2; h++)
+                    ptx::tmem_ld16(tbase + lane_off + (uint32_t)db * RT_NJ + (uint32_t)(g * RT_XJ + 16 * h), v[h]);
+                ptx::tmem_wait_ld();
+                // (x - xh)^2 in FP32 over 16 columns; x^2 in FP64 (exact
+                // products of FP32 values), so ||X||^2 matches an FP64 sum;
+                // four chains each
 #pragma unroll
-            for (int s = 0; s < RT_NJ / RT_XJ; s++, xi++) {
-                const int slot = (int)(xi % a.xs);
-                if (!*abort) ptx::mbar_wait(&sm.x_full[slot], (uint32_t)((xi / a.xs) & 1), abort);
-                if (!__all_sync(0xffffffffu, *abort == 0)) {
-                    stop = true;
-                    break;
+                for (int h = 0; h < 2; h++) {
+                    float fr[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int jj = 0; jj < 16; jj++) {
+                        const float x = xs[(16 * h + jj) * RT_ROWS];
+                        const float dv = x - __uint_as_float(v[h][jj]);
+                        fr[jj & 3] = fmaf(dv, dv, fr[jj & 3]);
+                        if (a.need_x2) sx[jj & 3] = fma((double)x, (double)x, sx[jj & 3]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; c++) sr[c] += (double)fr[c];
                 }
-                const float *xs = reinterpret_cast<const float *>(xring + (size_t)slot * RT_XBYTES) + hcol * RT_ROWS;
-                // (x - xh)^2 per tile in FP32; x^2 in FP64 (exact products of
-                // FP32 values), so ||X||^2 matches an FP64 sum; four chains
-                // each.  (FP32 tile sums for x^2 too measured 10 % faster at
-                // 512^3 R64 -- 0.159 against 0.176 ms -- for a 1e-9 error.)
-                float fr[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int jj = 0; jj < RT_XJ / 2; jj++) {
-                    const float x = xs[jj * RT_ROWS + row];
-                    const float dv = x - __uint_as_float(v[s][jj]);
-                    fr[jj & 3] = fmaf(dv, dv, fr[jj & 3]);
-                    if (a.need_x2) sx[jj & 3] = fma((double)x, (double)x, sx[jj & 3]);
-                }
-#pragma unroll
-                for (int c = 0; c < 4; c++) sr[c] += (double)fr[c];
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&sm.x_empty[slot]);
+                ptx::tc_fence_before();
             }
-            if (stop) break;
-            ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&sm.d_free[db]);
+            if (lane == 0) {
+                if (mine) ptx::mbar_arrive(&sm.x_empty[xr.slot]);
+                ptx::mbar_arrive(&sm.d_free[db]);
+            }
+            xr.next(tiles);
+            if (++q == a.nq) q = 0;
         }
         s_res = (sr[0] + sr[1]) + (sr[2] + sr[3]);
         s_x = (sx[0] + sx[1]) + (sx[2] + sx[3]);
@@ -346,8 +379,8 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
             s_x += __shfl_xor_sync(0xffffffffu, s_x, o);
         }
         if (lane == 0) {
-            sm.red[0][warp - 6] = s_res;
-            sm.red[1][warp - 6] = s_x;
+            sm.red[0][warp - 2 - RT_BLD] = s_res;
+            sm.red[1][warp - 2 - RT_BLD] = s_x;
         }
     }
 
@@ -374,6 +407,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
         a.part[2 * blockIdx.x] = r;
         a.part[2 * blockIdx.x + 1] = x;
     }
+    ptx::griddep_launch();
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 rt_encode_fn() {
