@@ -91,6 +91,10 @@ struct KrFactors {
 size_t mttkrp_ffma_ws_bytes(int order, const long *dims, int mode, long R, int round);
 int mttkrp_ffma(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,
                 int round, void *ws, cudaStream_t s);
+// Small tensors in one launch, plain FP32 (mttkrp_small.cu); no workspace.
+bool mttkrp_small_applies(int order, const long *dims, int mode, long R);
+int mttkrp_small(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,
+                 cudaStream_t s);
 // The MTTKRP on FP64 data (mttkrp_f64.cu); ws as sized here.
 size_t mttkrp_f64_ws_bytes(int order, const long *dims, int mode, long R);
 int mttkrp_f64(const double *X, int order, const long *dims, const double *const *U, int mode, long R,
@@ -98,6 +102,8 @@ int mttkrp_f64(const double *X, int order, const long *dims, const double *const
 // Tensor-core path (mttkrp_tc.cu): CUD_OK and the workspace size when it
 // applies to this shape/precision, CUD_ERR_UNSUPPORTED otherwise.
 int mttkrp_tc_query(int order, const long *dims, int mode, long R, int precision, size_t *ws_bytes);
+// Whether that path would run its packed-B kernel.
+bool mttkrp_tc_packed(int order, const long *dims, int mode, long R, int precision);
 // Where an MTTKRP left its result: M(q, r) = the sum over z < splits of
 // part[z zs + q qs + r rs], taken in FP64 in z order, or NaN everywhere when
 // *error is set (a CTA whose bounded wait expired).

@@ -4,6 +4,7 @@
 // tcgen05 tensor-core kernel where it applies (shape, alignment, rank) and
 // otherwise the CUDA-core kernel with the same operand rounding
 // (BF16X3/DEFAULT fall back to plain FP32, which is at least as accurate).
+// DEFAULT takes whichever of the two is faster.
 // The CUDA-core kernel of the entry points is mttkrp_ffma.cu's; a CP-ALS
 // plan's sweeps keep mttkrp_simt.cu's (see there).
 #include "kernels.cuh"
@@ -71,6 +72,30 @@ int sum_splits(const float *part, int splits, long Q, long R, long Rp, const int
     return CUD_OK;
 }
 
+namespace {
+
+// Small tensors run in plain FP32, which is what CUD_PREC_FP32 asks for and
+// at least as accurate as what CUD_PREC_DEFAULT promises.
+bool small_path(int order, const long *dims, int mode, long R, int precision) {
+    return (precision == CUD_PREC_FP32 || precision == CUD_PREC_DEFAULT) && mttkrp_small_applies(order, dims, mode, R);
+}
+
+// CUD_PREC_DEFAULT picks the faster of the tensor cores (BF16x3) and plain
+// FP32, never the less accurate one where they tie.  The tensor cores are
+// faster where the packed-B kernel runs, above 6.5e7 multiply-adds (B200, us a
+// mode, tensor cores / FP32: 160^3 R = 16 16.5 / 16.5, R = 32 17.0 / 22.0, 128^3
+// R = 32 16.3 / 13.7, R = 64 16.4 / 18.2, 256^3 R = 8 22.9 / 34.2); where the
+// Khatri-Rao rows are built per stage they are the slower ones (200^3 R = 16
+// 52 / 22, R = 64 105 / 48, 500^3 R = 32 704 / 248, 100^4 R = 16 512 / 164).
+bool default_fp32(int order, const long *dims, int mode, long R, int precision) {
+    if (precision != CUD_PREC_DEFAULT) return false;
+    double work = (double)R;
+    for (int m = 0; m < order; m++) work *= (double)dims[m];
+    return work <= 6.5e7 || !mttkrp_tc_packed(order, dims, mode, R, precision);
+}
+
+}  // namespace
+
 // Sized for both paths, so a call may fall back (e.g. a misaligned X) with
 // the same workspace.
 size_t mttkrp_ws_bytes(int order, const long *dims, int mode, long R, int precision) {
@@ -83,7 +108,8 @@ size_t mttkrp_ws_bytes(int order, const long *dims, int mode, long R, int precis
 
 int mttkrp_run(const float *X, int order, const long *dims, const float *const *U, int mode, long R,
                float *out, int precision, void *ws, cudaStream_t s) {
-    if (precision != CUD_PREC_FP32) {
+    if (small_path(order, dims, mode, R, precision)) return mttkrp_small(X, order, dims, U, mode, R, out, s);
+    if (precision != CUD_PREC_FP32 && !default_fp32(order, dims, mode, R, precision)) {
         size_t b = 0;
         if (mttkrp_tc_query(order, dims, mode, R, precision, &b) == CUD_OK) {
             int st = mttkrp_tc(X, order, dims, U, mode, R, out, precision, ws, s);
@@ -137,6 +163,9 @@ extern "C" int cud_mttkrp(const float *X, int order, const long *dims, const flo
 extern "C" int cud_mttkrp_path(int order, const long *dims, int mode, long R, int precision) {
     if (order < 2 || order > kMaxOrder || !dims || mode < 0 || mode >= order || R <= 0) return 0;
     if (precision == CUD_PREC_FP32) return 0;
+    for (int m = 0; m < order; m++)
+        if (dims[m] <= 0) return 0;
+    if (small_path(order, dims, mode, R, precision) || default_fp32(order, dims, mode, R, precision)) return 0;
     size_t b = 0;
     return mttkrp_tc_query(order, dims, mode, R, precision, &b) == CUD_OK ? 1 : 0;
 }

@@ -1343,6 +1343,11 @@ int mttkrp_tc_query(int order, const long *dims, int mode, long R, int precision
     return CUD_OK;
 }
 
+bool mttkrp_tc_packed(int order, const long *dims, int mode, long R, int precision) {
+    TcPlan p;
+    return tc_plan(order, dims, mode, R, precision, p) && p.pb;
+}
+
 int mttkrp_tc(const float *X, int order, const long *dims, const float *const *U, int mode, long R,
               float *out, int precision, void *ws, cudaStream_t s, MttkrpParts *parts) {
     TcPlan p;
