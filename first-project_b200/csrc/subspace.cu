@@ -18,6 +18,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "jacobi.cuh"
 #include "kernels.cuh"
 
 namespace cud {
@@ -28,20 +29,32 @@ namespace {
 
 constexpr int SI_RMAX = 64;
 
+// C (8 x 8) += A (8 x 4) B (4 x 8) in FP64.
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
 __device__ __forceinline__ unsigned long long si_mix(unsigned long long z) {
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
     return z ^ (z >> 31);
 }
 
-// V (n x r) = i.i.d. standard normal (Box-Muller over a counter hash).
+// Entry e of the start block: i.i.d. standard normal (Box-Muller over a
+// counter hash).
+__device__ __forceinline__ double si_start(long e) {
+    const double u1 = 1.0 - (double)(si_mix(2 * e + 0x51) >> 11) * (1.0 / 9007199254740992.0);
+    const double u2 = (double)(si_mix(2 * e + 0x52) >> 11) * (1.0 / 9007199254740992.0);
+    return sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
+}
+
+// V (n x r) = the start block.
 __global__ void k_si_init(double *V, long n, int r) {
     const long total = n * r;
-    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-        const double u1 = 1.0 - (double)(si_mix(2 * e + 0x51) >> 11) * (1.0 / 9007199254740992.0);
-        const double u2 = (double)(si_mix(2 * e + 0x52) >> 11) * (1.0 / 9007199254740992.0);
-        V[e] = sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
-    }
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x)
+        V[e] = si_start(e);
 }
 
 // V (n x r) = the given FP32 start block.
@@ -222,7 +235,8 @@ __global__ void __launch_bounds__(256) k_si_ritz(const double *V, const double *
 }
 
 // ---------------------------------------------------------------- fast path
-// r <= 32 and n <= 2048.  One step is two launches of the product G V
+// r <= 32 and n <= 2048, where the iteration does not fit in one launch
+// (k_si_run_cl).  One step is two launches of the product G V
 // (k_si_apply_cols; the k range split in slices whose partial products are
 // kept apart) and one launch of a cluster of CL_N CTAs that owns the n x r
 // iterate by row blocks (k_si_orth_cl): the partial products summed in
@@ -279,64 +293,64 @@ __device__ void cl_load_rows(const double *__restrict__ src, int nks, long n, in
     }
 }
 
+// Tile (ta, tb) of nt x nt (nt <= 4), or of its lower triangle in row order
+// when sym; without divisions, which a chain this short would feel.
 __device__ __forceinline__ void cl_tile(int tile, int nt, bool sym, int &ta, int &tb) {
-    if (sym) {  // lower-triangle tiles in row order
-        ta = 0;
-        int rem = tile;
-        while (rem > ta) {
-            rem -= ta + 1;
-            ta++;
-        }
-        tb = rem;
+    if (sym) {
+        ta = (tile >= 1) + (tile >= 3) + (tile >= 6);
+        tb = tile - (ta * (ta + 1) >> 1);
     } else {
-        ta = tile / nt;
+        ta = nt == 3 ? tile * 11 >> 5 : tile >> (nt >> 1);
         tb = tile - ta * nt;
     }
 }
 
 // out (32 x 32 row-major) = this CTA's rows' part of A^T B (lower triangle
-// when sym, with the diagonal tiles whole): 4 x 4 tiles, the rows split in
-// groups whose partials are added in group order.  Ends on a block barrier.
+// when sym, with the diagonal tiles whole): 8 x 8 tiles by FP64 matrix
+// instructions, the rows in 8, 2 or 1 groups for r <= 8, 16 or 32, whose
+// partials are added in group order.  gp: 1024 doubles.  Ends on a block
+// barrier.  (4 x 4 tiles a thread by FMAs took 2400 clocks for 32 rows and
+// r = 16, most of them bank conflicts between the partials; this takes 730.)
 __device__ void cl_cross(const double *A, const double *B, int nl, int r, bool sym, double *gp, double *out) {
-    const int nt = (r + 3) / 4;
-    const int ntiles = sym ? nt * (nt + 1) / 2 : nt * nt;
-    const int ng = min(8, CL_T / ntiles);
-    if ((int)threadIdx.x < ntiles * ng) {
-        const int tile = threadIdx.x % ntiles, g = threadIdx.x / ntiles;
-        int ta, tb;
-        cl_tile(tile, nt, sym, ta, tb);
-        const int i0 = g * nl / ng, i1 = (g + 1) * nl / ng;
-        double acc[4][4];
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int v = 0; v < 4; v++) acc[u][v] = 0.0;
-        for (int i = i0; i < i1; i++) {
-            const double *ra = A + i * CL_RS + 4 * ta, *rb = B + i * CL_RS + 4 * tb;
-            double xa[4], xb[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                xa[u] = ra[u];
-                xb[u] = rb[u];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int v = 0; v < 4; v++) acc[u][v] = fma(xa[u], xb[v], acc[u][v]);
+    constexpr int NW = CL_T / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nt = (r + 7) >> 3;
+    const int ntiles = sym ? nt * (nt + 1) >> 1 : nt * nt;
+    const int lg = nt == 1 ? 3 : nt == 2 ? 1 : 0, nk = (nl + 3) >> 2;
+    for (int it = w; it < ntiles << lg; it += NW) {
+        int g = 0, tile = it, ta, tb;
+        if (nt == 1) {
+            g = it;
+            tile = 0;
+        } else if (it >= ntiles) {
+            g = 1;
+            tile = it - ntiles;
         }
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int v = 0; v < 4; v++) gp[(g * ntiles + tile) * 16 + 4 * u + v] = acc[u][v];
+        cl_tile(tile, nt, sym, ta, tb);
+        double acc[2] = {0.0, 0.0};
+        const int k0 = g * nk >> lg, k1 = (g + 1) * nk >> lg;
+        int i = 4 * k0 + (lane & 3);
+        const double *pa = A + i * CL_RS + 8 * ta + (lane >> 2), *pb = B + i * CL_RS + 8 * tb + (lane >> 2);
+#pragma unroll 4
+        for (int k = k0; k < k1; k++) {
+            const bool in = i < nl;
+            dmma(acc, in ? *pa : 0.0, in ? *pb : 0.0);
+            i += 4;
+            pa += 4 * CL_RS;
+            pb += 4 * CL_RS;
+        }
+        double *o = gp + it * 64 + (lane >> 2) * 8 + 2 * (lane & 3);
+        o[0] = acc[0];
+        o[1] = acc[1];
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < ntiles * 16; e += CL_T) {
-        const int tile = e >> 4, u = (e >> 2) & 3, v = e & 3;
+    for (int e = threadIdx.x; e < ntiles * 64; e += CL_T) {
+        const int tile = e >> 6, u = (e >> 3) & 7, v = e & 7;
         int ta, tb;
         cl_tile(tile, nt, sym, ta, tb);
         double t = 0.0;
-        for (int g = 0; g < ng; g++) t += gp[(g * ntiles + tile) * 16 + 4 * u + v];
-        out[(4 * ta + u) * 32 + 4 * tb + v] = t;
+        for (int g = 0; g < 1 << lg; g++) t += gp[(g * ntiles + tile) * 64 + 8 * u + v];
+        out[(8 * ta + u) * 32 + 8 * tb + v] = t;
     }
     __syncthreads();
 }
@@ -345,132 +359,183 @@ __device__ void cl_cross(const double *A, const double *B, int nl, int r, bool s
 // buffer `red` (entries a, b < r, a >= b when sym; zero elsewhere).  The
 // caller has synchronised the cluster after the buffers were written.
 __device__ void cl_sum(cg::cluster_group &cl, double *red, int r, bool sym, double *dst) {
-    for (int e = threadIdx.x; e < 32 * 32; e += CL_T) {
-        const int a = e >> 5, b = e & 31;
-        double t = 0.0;
-        if (a < r && b < r && (!sym || a >= b))
-            for (int q = 0; q < CL_N; q++) t += cl.map_shared_rank(red, q)[e];
+    const int b = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const double *peer[CL_N];
+#pragma unroll
+    for (int q = 0; q < CL_N; q++) peer[q] = cl.map_shared_rank(red, q) + threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < 32 * 32 / CL_T; u++) {
+        const int a = w + (CL_T / 32) * u;
+        double v[CL_N], t = 0.0;
+        if (a < r && b < r && (!sym || a >= b)) {  // the loads go out together
+#pragma unroll
+            for (int q = 0; q < CL_N; q++) v[q] = peer[q][CL_T * u];
+#pragma unroll
+            for (int q = 0; q < CL_N; q++) t += v[q];
+        }
         dst[a * CL_RS + b] = t;
     }
     __syncthreads();
 }
 
-// CholQR's r x r factor work on all threads: C (lower triangle valid, in
-// shared memory) = L D L^T with unit L by right-looking elimination, and in
-// the same steps R = L^-1 (row k of R is final once step k-1 is done);
-// then T = (L D^1/2)^-1 = D^-1/2 R (32 x 32, zero outside the lower r x r
-// triangle).  Thread t keeps the cells (t / 32 + 8q, t % 32), q < 4, in
-// registers; step k's pivot column and row k of R are published through
-// shared memory, double-buffered, so a step takes one block barrier (a
-// sequential loop through shared memory would wait on every load).
-// Returns on every thread whether every pivot was positive and finite.
-__device__ __forceinline__ bool cl_chol_inv(const double *C, double *T, int r, double *pub, double *dsh) {
-    const int x = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double a[4], rr[4];
+// CholQR's r x r factor work: C (lower triangle valid, in shared memory) =
+// L D L^T with unit L, and R = L^-1, by eliminating the rows of [C | I] in
+// place: at step k column k of C is done and its place takes column k of R,
+// so a row i > k loses the same multiple of row k in every column.  Then
+// T = (L D^1/2)^-1 = D^-1/2 R (XL x XL, zero outside the lower r x r
+// triangle).  XL lanes to a row, NQ rows a thread (rows i = i0 + 8q): a step
+// reads row k, published in shared memory (double-buffered) with the pivot
+// in it, takes a_ik from lane k and ends on one barrier of the warps that
+// work.  A serial chain of the pivot's reciprocal, a product and an FMA, and
+// the issue slots of its warps: for r <= 16 four warps of two 16-lane rows
+// each.  16 steps took 16 000 clocks when C and R were two cases of a
+// branch, 3900 now.  Returns on every thread whether every pivot was positive
+// and finite.
+template <int XL>
+__device__ __forceinline__ bool cl_chol_steps(const double *C, double *T, int r, double *pub, double *dsh) {
+    constexpr int NQ = XL / 8, NTH = 8 * XL;  // 8 rows at a time
+    const int x = threadIdx.x % XL, i0 = threadIdx.x / XL, src = threadIdx.x & 31 & ~(XL - 1);
+    double v[NQ];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int i = w + 8 * q;
-        a[q] = (i < r && x < r && i >= x) ? C[i * CL_RS + x] : 0.0;
-        rr[q] = (i == x) ? 1.0 : 0.0;
-        if (x == 0 && i < r) pub[i] = a[q];  // column 0, buffer 0
+    for (int q = 0; q < NQ; q++) {
+        const int i = i0 + 8 * q;
+        v[q] = (i < r && x < r) ? C[max(i, x) * CL_RS + min(i, x)] : 0.0;
     }
-    __syncthreads();
+    if (i0 == 0) pub[x] = v[0];
+    asm volatile("bar.sync 1, %0;" ::"n"(NTH) : "memory");
     bool ok = true;
     for (int k = 0; k < r; k++) {
-        const double *col = pub + 64 * (k & 1), *row = col + 32;
-        double *ncol = pub + 64 * ((k + 1) & 1), *nrow = ncol + 32;
-        const double akk = col[k];
-        const bool good = akk > 0.0 && isfinite(akk);
-        ok = ok && good;
-        const double inv = good ? 1.0 / akk : 0.0;
-        if (threadIdx.x == 0) dsh[k] = good ? akk : 1.0;
-        const double cx = (x > k && x < r) ? col[x] * inv : 0.0;
-        const double rx = (x < k) ? row[x] : 1.0;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int i = w + 8 * q;
-            if (i < r && x < r) {
-                if (x > k && i >= x) a[q] = fma(-col[i], cx, a[q]);                // a_ix -= a_ik a_xk / a_kk
-                else if (i > k && x <= k) rr[q] = fma(-col[i] * inv, rx, rr[q]);   // R_ix -= (a_ik / a_kk) R_kx
-                if (x == k + 1 && i >= k + 1) ncol[i] = a[q];
-                if (i == k + 1 && x <= k) nrow[x] = rr[q];
-            }
+        const double *row = pub + 32 * (k & 1);
+        double *nrow = pub + 32 * ((k + 1) & 1);
+        const double akk = row[k];
+        double rx = row[x];
+        // 1 / a_kk = y (1 + f): the 20-bit estimate and a third-order Newton
+        // step, which the products with y do not wait for; the division where
+        // the estimate would flush or underflow
+        double y = rcp_approx(akk), f;
+        if ((unsigned)__double2hiint(akk) - 0x00100000u < 0x7e000000u) {
+            const double e = fma(-akk, y, 1.0);
+            f = fma(e, e, e);
+        } else {
+            const bool good = akk > 0.0 && isfinite(akk);
+            ok = ok && good;
+            y = good ? 1.0 / akk : 0.0;
+            f = 0.0;
         }
-        __syncthreads();
-    }
+        if (threadIdx.x == 0) dsh[k] = akk;
+        rx = (x == k ? 1.0 : rx) * y;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int i = w + 8 * q;
-        T[i * CL_RS + x] = (i < r && x <= i) ? rr[q] / sqrt(dsh[i]) : 0.0;
+        for (int q = 0; q < NQ; q++) {
+            const int i = i0 + 8 * q;
+            const double aik = __shfl_sync(0xffffffffu, v[q], src + k);
+            const double g = aik * rx;
+            const double t = fma(-g, f, fma(-aik, rx, x == k ? 0.0 : v[q]));
+            v[q] = i > k ? t : v[q];
+            if (i == k + 1) nrow[x] = t;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(NTH) : "memory");
     }
-    __syncthreads();
+    if (threadIdx.x < 32) dsh[threadIdx.x] = threadIdx.x < r ? 1.0 / sqrt(dsh[threadIdx.x]) : 0.0;
+    asm volatile("bar.sync 1, %0;" ::"n"(NTH) : "memory");
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+        const int i = i0 + 8 * q;
+        T[i * CL_RS + x] = (i < r && x <= i) ? (x == i ? 1.0 : v[q]) * dsh[i] : 0.0;
+    }
     return ok;
 }
 
-// dst[i][a] = sum_k M[a][k] src[i][k] over the nl rows (M 32 x 32, row
-// stride CL_RS; its zero rows beyond r keep dst's padding columns zero).
-// Four threads per row, eight outputs each (a = s, s + 4, ...).
-__device__ void cl_transform(const double *src, const double *M, int nl, double *dst) {
-    for (int it = threadIdx.x; it < nl * 4; it += CL_T) {
-        const int i = it >> 2, s = it & 3;
-        const double *y = src + i * CL_RS;
-        double acc[8];
+__device__ __forceinline__ bool cl_chol_inv(const double *C, double *T, int r, double *pub, double *dsh) {
+    __shared__ int s_ok;
+    if (r > 16) {
+        const bool ok = cl_chol_steps<32>(C, T, r, pub, dsh);
+        if (threadIdx.x == 0) s_ok = ok;
+    } else if (threadIdx.x < 128) {
+        const bool ok = cl_chol_steps<16>(C, T, r, pub, dsh);
+        if (threadIdx.x == 0) s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok;
+}
+
+// dst[i][a] = sum_k M[a][k] src[i][k] over the nl rows (M r x r, row stride
+// CL_RS, zero up to the next multiple of 8, as src's columns are), 8 x 8 tiles by FP64
+// matrix instructions; dst's columns up to the next multiple of 8 are zero.
+__device__ void cl_transform(const double *src, const double *M, int nl, int r, double *dst) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nt = (r + 7) >> 3, nk = (r + 3) >> 2;
+    for (int m = w; m < (nl + 7) >> 3; m += CL_T / 32) {
+        const int i = 8 * m + (lane >> 2);
+        const double *ps = src + i * CL_RS + (lane & 3), *pm = M + (lane >> 2) * CL_RS + (lane & 3);
+        double acc[4][2] = {};
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < 32; k++) {
-            const double yk = y[k];
+        for (int k = 0; k < 8; k++) {
+            if (k >= nk) break;
+            const double a = i < nl ? ps[4 * k] : 0.0;
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc[j] = fma(M[(s + 4 * j) * CL_RS + k], yk, acc[j]);
+            for (int j = 0; j < 4; j++)
+                if (j < nt) dmma(acc[j], a, pm[8 * j * CL_RS + 4 * k]);
         }
+        if (i < nl)
 #pragma unroll
-        for (int j = 0; j < 8; j++) dst[i * CL_RS + s + 4 * j] = acc[j];
+            for (int j = 0; j < 4; j++)
+                if (j < nt) {
+                    double *d = dst + i * CL_RS + 8 * j + 2 * (lane & 3);
+                    d[0] = acc[j][0];
+                    d[1] = acc[j][1];
+                }
     }
 }
 
-// Cyclic Jacobi on all threads (round-robin pairs, m/2 disjoint rotations
-// per round) on the symmetric H (r x r in Hs, row stride CL_RS), the
-// rotations accumulated in W.  Thread t keeps the cells (t / 32 + 8q,
-// t % 32), q < 4, of H and W in registers: a round's column rotations pair
-// lanes of one warp (shuffles), its row rotations read the partner row of
-// H J through shared memory (Mb).  Stops at a relative off-diagonal norm of
-// 1e-13 (rounding alone keeps it near r * eps, so a test at eps itself
-// would run every sweep).  On return Hs holds the rotated H, Ws = W (row
-// stride CL_RS) and ord the eigenvalue order, ascending.  Ends on a block
-// barrier.
-__device__ __forceinline__ void cl_jacobi(double *Hs, double *Mb, double *Ws, int r, double *cval, double *sval,
-                                          int *pt, int *role, int *ord, double *wred) {
-    const int x = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double h[4], wv[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int i = w + 8 * q;
-        h[q] = (i < r && x < r) ? 0.5 * (Hs[i * CL_RS + x] + Hs[x * CL_RS + i]) : 0.0;
-        wv[q] = (i == x && i < r) ? 1.0 : 0.0;
+// Cyclic Jacobi on all threads (round-robin pairs, h = m / 2 disjoint
+// rotations a round) on the symmetric part of H0 (r x r, row stride CL_RS,
+// zero beyond r), the rotations accumulated in W.  A round is a serial chain
+// of angles, update and one barrier: every warp forms the rotations itself
+// (lane k that of pair k) and a thread applies those of a pair of pairs to
+// their 2 x 2 cell of H, from one buffer into the other, or a pair's to one
+// row of W.  An odd r's dummy is a zero row, which no rotation touches.
+// The entries are read before the angles are formed, and warps without an
+// item form none (the angles' approximations share one unit).
+// Stops at a relative off-diagonal norm of 1e-13 (rounding alone keeps it
+// near r * eps, so a test at eps itself would run every sweep).  On return
+// ord is the eigenvalue order, ascending.  Ends on a block barrier.
+template <int NI>
+__device__ __forceinline__ void cl_jacobi(double *H0, double *H1, double *W, int r, int *ord, double *wred) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int h = (r + 1) / 2, m = 2 * h;
+    for (int e = tid; e < 32 * 32; e += CL_T) {
+        const int i = e >> 5, j = e & 31;
+        H1[i * CL_RS + j] = 0.5 * (H0[i * CL_RS + j] + H0[j * CL_RS + i]);
+        W[i * CL_RS + j] = (i == j && i < r) ? 1.0 : 0.0;
     }
-    if (threadIdx.x < 32) {  // unpaired indices rotate by the identity
-        pt[x] = x;
-        role[x] = 0;
-        cval[x] = 1.0;
-        sval[x] = 0.0;
-    }
-    __syncthreads();
+    // this thread's items: cells (k, l) of H first, then (pair k, row l) of W
+    // (NI of them: h (h + m) <= NI CL_T)
+    int ik[NI], il[NI];
+    bool cell[NI], has[NI];
 #pragma unroll
-    for (int q = 0; q < 4; q++) Hs[(w + 8 * q) * CL_RS + x] = h[q];
+    for (int u = 0; u < NI; u++) {
+        const int e = tid + CL_T * u, f = e - h * h;
+        cell[u] = f < 0;
+        has[u] = f < h * m;
+        ik[u] = cell[u] ? e / h : f % h;
+        il[u] = cell[u] ? e % h : has[u] ? f / h : 0;
+    }
+    const bool busy = __any_sync(0xffffffffu, has[0]);  // a warp without items only waits
     __syncthreads();
-    const int m = (r + 1) & ~1;
+    double *cur = H1, *nxt = H0;
     for (int sweep = 0; sweep < 40; sweep++) {
         double off = 0.0, tot = 0.0;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            tot = fma(h[q], h[q], tot);
-            if (w + 8 * q != x) off = fma(h[q], h[q], off);
+            const double v = cur[(w + 8 * q) * CL_RS + lane];
+            tot = fma(v, v, tot);
+            if (w + 8 * q != lane) off = fma(v, v, off);
         }
         for (int o = 16; o > 0; o >>= 1) {
             off += __shfl_xor_sync(0xffffffffu, off, o);
             tot += __shfl_xor_sync(0xffffffffu, tot, o);
         }
-        if (x == 0) {
+        if (lane == 0) {
             wred[w] = off;
             wred[8 + w] = tot;
         }
@@ -480,80 +545,127 @@ __device__ __forceinline__ void cl_jacobi(double *Hs, double *Mb, double *Ws, in
             o2 += wred[v];
             t2 += wred[8 + v];
         }
-        __syncthreads();  // wred is rewritten next sweep
-        if (o2 <= 1e-26 * t2) break;
+        if (o2 <= 1e-26 * t2) break;  // (a round's barrier comes before wred's next write)
         for (int round = 0; round < m - 1; round++) {
-            if ((int)threadIdx.x < m / 2) {
-                const int k = threadIdx.x;
-                const int a = (k == 0) ? m - 1 : (round + k) % (m - 1);
-                const int b = (k == 0) ? round % (m - 1) : (round + m - 1 - k) % (m - 1);
-                const int p = min(a, b), q = max(a, b);
-                double c = 1.0, sv = 0.0;
-                if (q < r) {
-                    const double hpq = Hs[p * CL_RS + q];
-                    if (hpq != 0.0) {
-                        const double theta = (Hs[q * CL_RS + q] - Hs[p * CL_RS + p]) / (2.0 * hpq);
-                        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                        c = 1.0 / sqrt(t * t + 1.0);
-                        sv = t * c;
+            if (busy) {
+                // pair k of the round: (m - 1, round) or (round + k, round - k) mod m - 1
+                int a = round + lane, b = round - lane;
+                if (a >= m - 1) a -= m - 1;
+                if (b < 0) b += m - 1;
+                if (lane == 0) a = m - 1;
+                const int p = min(a, b) * CL_RS, q = max(a, b) * CL_RS;
+                const int pc = min(a, b), qc = max(a, b), pq = pc | qc << 8;
+                const bool pair = lane < h;
+                const double app = pair ? cur[p + pc] : 1.0, aqq = pair ? cur[q + qc] : 1.0,
+                             apq = pair ? cur[p + qc] : 0.0;
+                int cq[NI];
+                double *d0[NI], *d1[NI], x[NI], y[NI], z[NI], t[NI];
+#pragma unroll
+                for (int u = 0; u < NI; u++) {  // the items' entries, ahead of the angles
+                    const int k = __shfl_sync(0xffffffffu, pq, ik[u]);
+                    const int l = __shfl_sync(0xffffffffu, pq, cell[u] ? il[u] : 0);
+                    const int pk = k & 255, qk = k >> 8, pl = l & 255, ql = l >> 8;
+                    const bool in_w = has[u] && !cell[u];
+                    d0[u] = in_w ? W + il[u] * CL_RS + pk : cur + pk * CL_RS + pl;
+                    d1[u] = in_w ? W + il[u] * CL_RS + qk : cur + qk * CL_RS + pl;
+                    cq[u] = ql - pl;
+                    x[u] = *d0[u];
+                    y[u] = *d1[u];
+                    z[u] = cell[u] ? d0[u][cq[u]] : 0.0;
+                    t[u] = cell[u] ? d1[u][cq[u]] : 0.0;
+                }
+                double c, s;
+                jacobi_rotation<false>(app, aqq, apq, c, s);
+#pragma unroll
+                for (int u = 0; u < NI; u++) {
+                    const double ck = __shfl_sync(0xffffffffu, c, ik[u]), sk = __shfl_sync(0xffffffffu, s, ik[u]);
+                    const double cl = __shfl_sync(0xffffffffu, c, cell[u] ? il[u] : 0),
+                                 sl = __shfl_sync(0xffffffffu, s, cell[u] ? il[u] : 0);
+                    const double x1 = ck * x[u] - sk * y[u], y1 = sk * x[u] + ck * y[u];
+                    if (cell[u]) {
+                        const double z1 = ck * z[u] - sk * t[u], t1 = sk * z[u] + ck * t[u];
+                        double *n0 = d0[u] + (nxt - cur), *n1 = d1[u] + (nxt - cur);
+                        n0[0] = cl * x1 - sl * z1;
+                        n0[cq[u]] = sl * x1 + cl * z1;
+                        n1[0] = cl * y1 - sl * t1;
+                        n1[cq[u]] = sl * y1 + cl * t1;
+                    } else if (has[u]) {
+                        *d0[u] = x1;
+                        *d1[u] = y1;
                     }
-                    pt[p] = q;
-                    pt[q] = p;
-                    role[q] = 1;
-                } else {
-                    pt[p] = p;
-                    pt[q] = q;
-                    role[q] = 0;
-                }
-                role[p] = 0;
-                cval[p] = c;
-                cval[q] = c;
-                sval[p] = sv;
-                sval[q] = sv;
-            }
-            __syncthreads();
-            {  // H J and W J: columns x and pt[x] live in lanes of the same warp
-                const int px = pt[x], rx = role[x];
-                const double cx = cval[x], sx = rx ? sval[x] : -sval[x];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const double ho = __shfl_sync(0xffffffffu, h[q], px);
-                    const double wo = __shfl_sync(0xffffffffu, wv[q], px);
-                    h[q] = fma(sx, ho, cx * h[q]);
-                    wv[q] = fma(sx, wo, cx * wv[q]);
-                    Mb[(w + 8 * q) * CL_RS + x] = h[q];
                 }
             }
             __syncthreads();
-#pragma unroll
-            for (int q = 0; q < 4; q++) {  // J^T (H J): row i against its partner row
-                const int i = w + 8 * q;
-                const int pi = pt[i];
-                const double ci = cval[i], si = role[i] ? sval[i] : -sval[i];
-                h[q] = fma(si, Mb[pi * CL_RS + x], ci * h[q]);
-                Hs[i * CL_RS + x] = h[q];
-            }
-            __syncthreads();
+            double *t = cur;
+            cur = nxt;
+            nxt = t;
         }
     }
-#pragma unroll
-    for (int q = 0; q < 4; q++) Ws[(w + 8 * q) * CL_RS + x] = wv[q];
-    if (threadIdx.x < 32) {  // ascending order by rank (ties by index); a
-                             // non-permutation (NaN eigenvalues) falls back
-                             // to the identity order
+    if (tid < 32) {  // ascending order by rank (ties by index); a
+                     // non-permutation (NaN eigenvalues) falls back
+                     // to the identity order
         int rk = 0;
-        if (x < r) {
-            const double d = Hs[x * CL_RS + x];
+        if (lane < r) {
+            const double d = cur[lane * CL_RS + lane];
             for (int b = 0; b < r; b++) {
-                const double e = Hs[b * CL_RS + b];
-                rk += (e < d) || (e == d && b < x);
+                const double e = cur[b * CL_RS + b];
+                rk += (e < d) || (e == d && b < lane);
             }
         }
-        const unsigned bits = __reduce_or_sync(0xffffffffu, x < r ? 1u << rk : 0u);
+        const unsigned bits = __reduce_or_sync(0xffffffffu, lane < r ? 1u << rk : 0u);
         const unsigned want = (r == 32) ? 0xffffffffu : ((1u << r) - 1u);
-        if (x < r) ord[bits == want ? rk : x] = x;
+        if (lane < r) ord[bits == want ? rk : lane] = lane;
     }
     __syncthreads();
+}
+
+// Two CholQR passes on the cluster's row blocks, ya -> yb -> ya; false, in
+// every CTA, when a Gram is not numerically positive definite.
+__device__ __forceinline__ bool cl_orth(cg::cluster_group &cl, double *ya, double *yb, int nl, int r, double *red,
+                                        double *gp, double *C, double *T, double *pub, double *dsh) {
+    for (int pass = 0; pass < 2; pass++) {
+        double *src = pass ? yb : ya, *dst = pass ? ya : yb, *rb = red + pass * 32 * 32;
+        cl_cross(src, src, nl, r, true, gp, rb);
+        cl.sync();
+        cl_sum(cl, rb, r, true, C);
+        if (!cl_chol_inv(C, T, r, pub, dsh)) return false;
+        cl_transform(src, T, nl, r, dst);
+        __syncthreads();
+    }
+    return true;
+}
+
+// r - ||C||_F^2 (32 x 32, row stride CL_RS), on every thread.
+__device__ __forceinline__ double cl_gap(const double *C, int r, double *wred) {
+    double t = 0.0;
+    for (int e = threadIdx.x; e < 32 * 32; e += CL_T) {
+        const double v = C[(e >> 5) * CL_RS + (e & 31)];
+        t = fma(v, v, t);
+    }
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = t;
+    __syncthreads();
+    double g = 0.0;
+    for (int w = 0; w < CL_T / 32; w++) g += wred[w];
+    __syncthreads();
+    return (double)r - g;
+}
+
+// V w_ord[j], ascending: the columns of W in M[j][a] = W[a][ord[j]], then
+// dst = src M^T, and this CTA's rows of U.
+__device__ __forceinline__ void cl_ritz_out(const double *src, const double *W, const int *ord, double *M, double *dst,
+                                            int nl, int r, long i0, long n, float *__restrict__ U) {
+    for (int e = threadIdx.x; e < 32 * 32; e += CL_T) {
+        const int j = e >> 5, a = e & 31;
+        M[j * CL_RS + a] = (j < r && a < r) ? W[a * CL_RS + ord[j]] : 0.0;
+    }
+    __syncthreads();
+    cl_transform(src, M, nl, r, dst);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nl * r; e += CL_T) {
+        const int j = e / nl, i = e - j * nl;
+        U[(i0 + i) + n * j] = (float)dst[i * CL_RS + j];
+    }
 }
 
 // Y (n x r) = orth(sum of the nks partial slices) by two CholQR passes;
@@ -582,21 +694,13 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
            *T = smc + L.T;
     cl_load_rows(part, nks, n, r, i0, nl, ya);
     __syncthreads();
-    for (int pass = 0; pass < 2; pass++) {
-        double *src = pass ? yb : ya, *dst = pass ? ya : yb, *rb = red + pass * 32 * 32;
-        cl_cross(src, src, nl, r, true, gp, rb);
-        cl.sync();
-        cl_sum(cl, rb, r, true, C);
-        if (!cl_chol_inv(C, T, r, pub, dsh)) {  // the same verdict in every CTA
-            cl.sync();                              // peers may still read this CTA's buffers
-            if (rank == 0 && threadIdx.x == 0) {
-                *fail = 1;
-                if (st) st[0] = 1;
-            }
-            return;
+    if (!cl_orth(cl, ya, yb, nl, r, red, gp, C, T, pub, dsh)) {  // the same verdict in every CTA
+        cl.sync();                                                  // peers may still read this CTA's buffers
+        if (rank == 0 && threadIdx.x == 0) {
+            *fail = 1;
+            if (st) st[0] = 1;
         }
-        cl_transform(src, T, nl, dst);
-        __syncthreads();
+        return;
     }
     if (Vold) {
         cl_load_rows(Vold, 1, n, r, i0, nl, yb);
@@ -605,19 +709,8 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
         cl.sync();
         if (rank == 0) {
             cl_sum(cl, red, r, false, C);
-            double t = 0.0;
-            for (int e = threadIdx.x; e < 32 * 32; e += CL_T) {
-                const double v = C[(e >> 5) * CL_RS + (e & 31)];
-                t = fma(v, v, t);
-            }
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = t;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double g = 0.0;
-                for (int w = 0; w < CL_T / 32; w++) g += wred[w];
-                scal[0] = (double)r - g;
-            }
+            const double g = cl_gap(C, r, wred);
+            if (threadIdx.x == 0) scal[0] = g;
         }
     }
     for (int e = threadIdx.x; e < nl * r; e += CL_T) {
@@ -646,8 +739,8 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
                  float *__restrict__ U) {
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ double smc[];
-    __shared__ double cval[32], sval[32], wred[16];
-    __shared__ int pt[32], role[32], ord[32];
+    __shared__ double wred[16];
+    __shared__ int ord[32];
     const ClLayout L = cl_layout(n);
     const int rank = (int)cl.block_rank();
     const long i0 = (long)rank * L.nl;
@@ -660,19 +753,204 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
     cl_cross(yb, ya, nl, r, false, gp, red);
     cl.sync();
     cl_sum(cl, red, r, false, H);
-    cl_jacobi(H, gp, W, r, cval, sval, pt, role, ord, wred);
-    double *M = gp + 32 * CL_RS;  // M[j][a] = W[a][ord[j]]
-    for (int e = threadIdx.x; e < 32 * 32; e += CL_T) {
-        const int j = e >> 5, a = e & 31;
-        M[j * CL_RS + a] = (j < r && a < r) ? W[a * CL_RS + ord[j]] : 0.0;
+    cl_jacobi<3>(H, gp, W, r, ord, wred);
+    cl_ritz_out(yb, W, ord, gp + 32 * CL_RS, ya, nl, r, i0, n, U);
+    cl.sync();  // keep this CTA's buffers alive until every peer has read them
+}
+
+// ------------------------------------------------- the iteration in one launch
+// Where an eighth of G fits in a CTA's shared memory beside two copies of V,
+// one cluster keeps G there (its rows, as the iterate's) and runs the whole
+// iteration: start block, steps, Rayleigh-Ritz.  The n x r products are FP64
+// matrix instructions on shared memory; each CTA sends its rows of the
+// result to its peers' copies (distributed shared memory), so a step waits
+// on four cluster barriers.  Bound by the serial chain of the r x r work
+// between them.  B200, each of the three modes of a 256^3 rank-16 HOSVD:
+// 260 us of kernels, and the gaps between 11 launches, with a launch per
+// product and per orthonormalisation; 105 us here (the whole call 1333 us,
+// now 782).
+
+// Dynamic shared memory (offsets in doubles): G's rows (padded to eights, row
+// stride ldg), the two copies of V (row-major, row stride ldv; the second
+// also holds the tile partials of the r x r work, which needs it between two
+// products only), then as ClLayout.  ldg and ldv are 4 mod 8, so that the
+// fragments' four rows or columns fall in different banks.
+struct RunLayout {
+    int nl, nlp, kp, ldg, ldv;
+    size_t va, vb, ya, yb, red, C, T, total;
+};
+__host__ __device__ inline RunLayout run_layout(long n, int nt) {
+    RunLayout L;
+    L.nl = (int)((n + CL_N - 1) / CL_N);
+    L.nlp = (L.nl + 7) / 8 * 8;
+    L.kp = (int)((n + 7) / 8 * 8);
+    L.ldg = L.kp + 4;
+    L.ldv = 8 * nt + 4;
+    const size_t v = (size_t)L.kp * L.ldv, gp = (size_t)CL_T * 16;
+    L.va = (size_t)L.nlp * L.ldg;
+    L.vb = L.va + v;
+    L.ya = L.vb + (v > gp ? v : gp);
+    L.yb = L.ya + (size_t)L.nl * CL_RS;
+    L.red = (L.yb + (size_t)L.nl * CL_RS + 1) / 2 * 2;
+    L.C = L.red + 2 * 32 * 32;
+    L.T = L.C + 32 * CL_RS;
+    L.total = L.T + 32 * CL_RS;
+    return L;
+}
+constexpr size_t RUN_SMEM_MAX = 224 * 1024;
+
+// out (nl x r, row stride CL_RS) = this CTA's rows of G V.  A warp takes 8
+// rows and a share of k, with two accumulator sets for the matrix
+// instructions' latency; the shares are added in order.  part: 32 x 64
+// doubles.  Ends on a block barrier.
+template <int NT>
+__device__ __forceinline__ void run_apply(const RunLayout &L, const double *G, const double *V, double *part,
+                                          double *out) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int mt = L.nlp / 8, ks = max(1, (CL_T / 32) / mt), nk = L.kp / 4;
+    for (int it = w; it < mt * ks; it += CL_T / 32) {
+        const int m = it % mt, s = it / mt;
+        const int k0 = s * nk / ks, k1 = (s + 1) * nk / ks;
+        double acc[2][NT][2];
+#pragma unroll
+        for (int j = 0; j < NT; j++) acc[0][j][0] = acc[0][j][1] = acc[1][j][0] = acc[1][j][1] = 0.0;
+        const double *g = G + (8 * m + (lane >> 2)) * L.ldg + (lane & 3) + 4 * k0;
+        const double *v = V + ((lane & 3) + 4 * k0) * L.ldv + (lane >> 2);
+        const int step = 4 * L.ldv;
+        int k = k0;
+#pragma unroll 4
+        for (; k + 1 < k1; k += 2) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const double a = *g;
+#pragma unroll
+                for (int j = 0; j < NT; j++) dmma(acc[u][j], a, v[8 * j]);
+                g += 4;
+                v += step;
+            }
+        }
+        if (k < k1) {
+            const double a = *g;
+#pragma unroll
+            for (int j = 0; j < NT; j++) dmma(acc[0][j], a, v[8 * j]);
+        }
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int x = 0; x < 2; x++)
+                part[((s * mt + m) * 8 + (lane >> 2)) * (8 * NT) + 8 * j + 2 * (lane & 3) + x] =
+                    acc[0][j][x] + acc[1][j][x];
     }
     __syncthreads();
-    cl_transform(yb, M, nl, ya);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nl * r; e += CL_T) {
-        const int j = e / nl, i = e - j * nl;
-        U[(i0 + i) + n * j] = (float)ya[i * CL_RS + j];
+    for (int e = threadIdx.x; e < L.nl * 8 * NT; e += CL_T) {
+        const int i = e / (8 * NT), c = e % (8 * NT);
+        double t = 0.0;
+        for (int s = 0; s < ks; s++) t += part[(s * mt * 8 + i) * (8 * NT) + c];
+        out[i * CL_RS + c] = t;
     }
+    __syncthreads();
+}
+
+// Every CTA's copy V (rows i0 .. i0 + nl - 1) = src.  The caller synchronises
+// the cluster.
+template <int NT>
+__device__ __forceinline__ void run_send(cg::cluster_group &cl, const RunLayout &L, const double *src, int nl, long i0,
+                                         double *V) {
+    for (int e = threadIdx.x; e < nl * 4 * NT; e += CL_T) {
+        const int i = e / (4 * NT), c = e % (4 * NT);
+        const double2 v = make_double2(src[i * CL_RS + 2 * c], src[i * CL_RS + 2 * c + 1]);
+        double *d = V + (i0 + i) * L.ldv + 2 * c;
+#pragma unroll
+        for (int q = 0; q < CL_N; q++) *reinterpret_cast<double2 *>(cl.map_shared_rank(d, q)) = v;
+    }
+}
+
+// state (pinned host memory): 1 converged, 2 not within max_iters, 3 a rank-
+// deficient iterate; U is written in the first case only.
+template <int NT>
+__global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
+    k_si_run_cl(const double *__restrict__ Gm, long n, int r, const float *U0, float *U, int max_iters,
+                volatile int *state) {
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) double smc[];
+    __shared__ double pub[128], dsh[32], wred[16];
+    __shared__ int ord[32];
+    const RunLayout L = run_layout(n, NT);
+    const int rank = (int)cl.block_rank();
+    const long i0 = (long)rank * L.nl;
+    const int nl = (int)max(0L, min((long)L.nl, n - i0));
+    double *G = smc, *va = smc + L.va, *vb = smc + L.vb, *gp = vb, *ya = smc + L.ya, *yb = smc + L.yb,
+           *red = smc + L.red, *C = smc + L.C, *T = smc + L.T;
+    // G's rows are on their way while the start block is orthonormalised
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = lane; i < L.nlp; i += 32)
+#pragma unroll 4
+        for (int k = w; k < L.kp; k += CL_T / 32) {
+            double *d = G + i * L.ldg + k;
+            if (i < nl && k < n)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(d)),
+                             "l"(Gm + (i0 + i) + n * k)
+                             : "memory");
+            else
+                *d = 0.0;
+        }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int e = threadIdx.x; e < (L.kp - (int)n) * L.ldv; e += CL_T) va[n * L.ldv + e] = 0.0;
+    for (int i = lane; i < L.nl; i += 32)
+        for (int a = w; a < CL_RS; a += CL_T / 32) {
+            const long x = (i0 + i) + n * a;
+            ya[i * CL_RS + a] = (i < nl && a < r) ? (U0 ? (double)U0[x] : si_start(x)) : 0.0;
+            yb[i * CL_RS + a] = 0.0;
+        }
+    __syncthreads();
+    int verdict = 0;  // the same in every CTA
+    if (!cl_orth(cl, ya, yb, nl, r, red, gp, C, T, pub, dsh)) verdict = 3;
+    run_send<NT>(cl, L, ya, nl, i0, va);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    cl.sync();
+    int extra = -1;  // steps still to run after the tolerance is met
+    for (int step = 0; verdict == 0; step++) {
+        if (step == max_iters) {
+            verdict = 2;
+            break;
+        }
+        // two products per orthonormalisation (G^2 V): the columns' condition
+        // grows by (lambda_1 / lambda_r)^2 per step, well inside CholQR2's range
+        run_apply<NT>(L, G, va, C, yb);
+        for (int e = threadIdx.x; e < (L.kp - (int)n) * L.ldv; e += CL_T) vb[n * L.ldv + e] = 0.0;
+        run_send<NT>(cl, L, yb, nl, i0, vb);
+        cl.sync();
+        run_apply<NT>(L, G, vb, C, ya);
+        if (!cl_orth(cl, ya, yb, nl, r, red, gp, C, T, pub, dsh)) {
+            verdict = 3;
+            break;
+        }
+        // the gap r - ||Vold^T V||^2, and V to the peers under the same barrier
+        for (int e = threadIdx.x; e < nl * 32; e += CL_T) {
+            const int i = e >> 5, a = e & 31;
+            yb[i * CL_RS + a] = (a < r) ? va[(i0 + i) * L.ldv + a] : 0.0;
+        }
+        __syncthreads();
+        cl_cross(yb, ya, nl, r, false, gp, red);
+        run_send<NT>(cl, L, ya, nl, i0, va);
+        cl.sync();
+        cl_sum(cl, red, r, false, C);
+        const double gap = cl_gap(C, r, wred);
+        // one more step after the gap first falls below the tolerance
+        if (extra < 0 && gap < 1e-13 * (double)r) extra = 1;
+        if (extra >= 0 && extra-- == 0) verdict = 1;
+    }
+    if (verdict == 1) {
+        // Rayleigh-Ritz on H = V^T (G V).  The second of the two buffers the
+        // peers read: the first may still be read for the gap.
+        run_apply<NT>(L, G, va, C, yb);
+        cl_cross(ya, yb, nl, r, false, gp, red + 32 * 32);
+        cl.sync();
+        cl_sum(cl, red + 32 * 32, r, false, C);
+        cl_jacobi<NT <= 2 ? 1 : NT - 1>(C, gp, T, r, ord, wred);
+        cl_ritz_out(ya, T, ord, gp + 32 * CL_RS, yb, nl, r, i0, n, U);
+    }
+    if (rank == 0 && threadIdx.x == 0) *state = verdict;
     cl.sync();  // keep this CTA's buffers alive until every peer has read them
 }
 
@@ -845,6 +1123,39 @@ cudaGraphExec_t si_loop_graph(int dev, const SiSteps &k, int max_iters) {
 
 size_t subspace_ws_doubles(long n, long r) { return 3 * (size_t)n * r + 8; }  // V, Y, W (r*r <= n*r), scalars
 
+// The whole iteration in one launch of a cluster (k_si_run_cl).
+// CUD_ERR_UNSUPPORTED when its shared memory or the cluster does not fit.
+template <int NT>
+static int top_eigvecs_run(const double *G, long n, long r, float *U, int max_iters, cudaStream_t s,
+                           const float *U0) {
+    const size_t smem = run_layout(n, NT).total * sizeof(double);
+    if (smem > RUN_SMEM_MAX) return CUD_ERR_UNSUPPORTED;
+    int dev = 0;
+    CUD_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return CUD_ERR_UNSUPPORTED;
+    static std::atomic<int> ready[64];  // 0 unknown, 1 usable, 2 not; zero-initialised
+    if (!ready[dev]) {
+        CUD_CHECK(cudaFuncSetAttribute(k_si_run_cl<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RUN_SMEM_MAX));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(CL_N);
+        cfg.blockDim = dim3(CL_T);
+        cfg.dynamicSmemBytes = RUN_SMEM_MAX;
+        int nc = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&nc, k_si_run_cl<NT>, &cfg);
+        ready[dev] = (e == cudaSuccess && nc > 0) ? 1 : 2;
+        (void)cudaGetLastError();
+    }
+    if (ready[dev] != 1) return CUD_ERR_UNSUPPORTED;
+    double *h = pinned_scalars();
+    if (!h) return CUD_ERR_NO_MEMORY;
+    volatile int *state = reinterpret_cast<volatile int *>(h);
+    *state = 0;
+    k_si_run_cl<NT><<<CL_N, CL_T, smem, s>>>(G, n, (int)r, U0, U, max_iters, state);
+    CUD_CHECK_LAUNCH("subspace iteration");
+    CUD_CHECK(cudaStreamSynchronize(s));
+    return *state == 1 ? CUD_OK : CUD_ERR_NOT_CONVERGED;
+}
+
 // Fast path (r <= 32, n <= 2048): ws holds V, Y (n x r each) and two sets
 // of nks partial products, nks as many as ws_doubles allows (at most 8).
 // Each step forms G^2 V (two split products), then orthonormalises and
@@ -927,6 +1238,13 @@ static int top_eigvecs_fast(const double *G, long n, long r, float *U, double *w
 
 static int subspace_run(const double *G, long n, long r, float *U, double *ws, size_t ws_doubles, int max_iters,
                         cudaStream_t s, const float *U0) {
+    if (r <= SI_FR) {
+        const int st = r <= 8    ? top_eigvecs_run<1>(G, n, r, U, max_iters, s, U0)
+                       : r <= 16 ? top_eigvecs_run<2>(G, n, r, U, max_iters, s, U0)
+                       : r <= 24 ? top_eigvecs_run<3>(G, n, r, U, max_iters, s, U0)
+                                 : top_eigvecs_run<4>(G, n, r, U, max_iters, s, U0);
+        if (st != CUD_ERR_UNSUPPORTED) return st;
+    }
     if (r <= SI_FR && n <= 2048 && cl_layout(n).total * sizeof(double) <= CL_SMEM_MAX) {
         const int st = top_eigvecs_fast(G, n, r, U, ws, ws_doubles, max_iters, s, U0);
         if (st != CUD_ERR_UNSUPPORTED) return st;
