@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
+#include "tc_ptx.cuh"
 
 namespace cud {
 
@@ -153,6 +154,8 @@ __global__ void k_take_top_f32(const double *__restrict__ V, long n, long r, flo
 }
 
 __global__ void k_to_bf16(const float *__restrict__ a, __nv_bfloat16 *__restrict__ b, long n) {
+    ptx::griddep_wait();
+    ptx::griddep_launch();
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x)
         b[e] = __float2bfloat16_rn(a[e]);
 }
@@ -162,6 +165,8 @@ unsigned gfor(long n) { return (unsigned)std::min<long>((n + 255) / 256, 16L * k
 // a (n floats) -> hi (bf16(a)) and lo (bf16(a - hi)).
 __global__ void k_split_bf16(const float *__restrict__ a, __nv_bfloat16 *__restrict__ hi,
                              __nv_bfloat16 *__restrict__ lo, long n) {
+    ptx::griddep_wait();
+    ptx::griddep_launch();
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x)
         put_split(hi, lo, e, a[e]);
 }
@@ -172,6 +177,8 @@ __global__ void k_split_bf16(const float *__restrict__ a, __nv_bfloat16 *__restr
 __global__ void k_ttm3_finish(const float *__restrict__ F2, const float *__restrict__ F3, long n,
                               float *__restrict__ fout, __nv_bfloat16 *__restrict__ hi,
                               __nv_bfloat16 *__restrict__ lo) {
+    ptx::griddep_wait();
+    ptx::griddep_launch();
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         const float v = (F2[e] + F2[e + n]) + F3[e];
         if (fout) fout[e] = v;
@@ -348,6 +355,8 @@ GemmEpi epi_f32(float *out, long ldm, long ldn, int accumulate) {
 // g64 = HH + P + P^T in FP64 (P = hi lo^T; its transpose is lo hi^T).
 __global__ void k_gram_finish(const float *__restrict__ HH, const float *__restrict__ P, long I,
                               double *__restrict__ g64) {
+    ptx::griddep_wait();
+    ptx::griddep_launch();
     const long n2 = I * I;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n2; e += (long)gridDim.x * blockDim.x) {
         const long m = e / I, n = e - m * I;
@@ -366,7 +375,8 @@ int gram_tc(const TcWork &w, long I, long K, bool use_lo, cudaStream_t s) {
     if (use_lo && w.ul) {
         float *P = reinterpret_cast<float *>(w.V);
         if ((st = gemm_tc_bf16(w.uh, K, w.ul, K, I, I, K, epi_f32(P, I, 1, 0), w.gws, s))) return st;
-        k_gram_finish<<<gfor(I * I), 256, 0, s>>>(w.g32, P, I, w.g64);
+        PdlLaunch l(gfor(I * I), 256, 0, s);
+        CUD_CHECK(cudaLaunchKernelEx(&l.cfg, k_gram_finish, (const float *)w.g32, (const float *)P, I, w.g64));
     } else {
         k_f32_to_f64<<<gfor(I * I), 256, 0, s>>>(w.g32, w.g64, I * I);
     }
@@ -397,8 +407,8 @@ int top_vectors(const TcWork &w, long I, long r, float *U, cudaStream_t s, bool 
 int ttm_fast(const TcWork &w, const __nv_bfloat16 *T, long K, long rest, const float *U, long r,
              __nv_bfloat16 *zout, float *fout, cudaStream_t s) {
     if (gemm_tc_ws_bytes(rest, r, K) > w.gws_bytes) return CUD_ERR_INVALID_ARGUMENT;
-    k_to_bf16<<<gfor(K * r), 256, 0, s>>>(U, w.ub, K * r);
-    CUD_CHECK_LAUNCH("ttm factor bf16");
+    PdlLaunch l(gfor(K * r), 256, 0, s);
+    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, k_to_bf16, U, w.ub, K * r));
     GemmEpi e;
     memset(&e, 0, sizeof(e));
     e.alpha = 1.f;
@@ -417,8 +427,8 @@ int ttm3_fast(const TcWork &w, const __nv_bfloat16 *Th, const __nv_bfloat16 *Tl,
               long r, __nv_bfloat16 *zh, __nv_bfloat16 *zl, float *fout, cudaStream_t s) {
     if (gemm_tc_ws_bytes(rest, 2 * r, K) > w.gws_bytes) return CUD_ERR_INVALID_ARGUMENT;
     const __nv_bfloat16 *Uh = w.ub, *Ul = w.ub + K * r;
-    k_split_bf16<<<gfor(K * r), 256, 0, s>>>(U, w.ub, w.ub + K * r, K * r);
-    CUD_CHECK_LAUNCH("ttm3 factor split");
+    PdlLaunch l(gfor(K * r), 256, 0, s);
+    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, k_split_bf16, U, w.ub, w.ub + K * r, K * r));
     int st;
     if (2 * r <= 32) {
         if ((st = gemm_tc_bf16(Th, K, Uh, K, rest, 2 * r, K, epi_f32(w.f2, 1, rest, 0), w.gws, s))) return st;
@@ -428,8 +438,8 @@ int ttm3_fast(const TcWork &w, const __nv_bfloat16 *Th, const __nv_bfloat16 *Tl,
             return st;
     }
     if ((st = gemm_tc_bf16(Tl, K, Uh, K, rest, r, K, epi_f32(w.f3, 1, rest, 0), w.gws, s))) return st;
-    k_ttm3_finish<<<gfor(rest * r), 256, 0, s>>>(w.f2, w.f3, rest * r, fout, zh, zl);
-    CUD_CHECK_LAUNCH("ttm3 finish");
+    PdlLaunch lf(gfor(rest * r), 256, 0, s);
+    CUD_CHECK(cudaLaunchKernelEx(&lf.cfg, k_ttm3_finish, (const float *)w.f2, (const float *)w.f3, rest * r, fout, zh, zl));
     return CUD_OK;
 }
 
