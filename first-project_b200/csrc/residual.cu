@@ -196,8 +196,8 @@ namespace {
 
 // ---------------------------------------------------------------------------
 // FFMA fast path (R <= 64, mode-0 rows a multiple of 4, U_1's rows a
-// multiple of 32, X and U_1 16-byte aligned): the SGEMM-style tile of the
-// plain FP32 MTTKRP, transposed.  A CTA owns RQ = 128 rows q of mode 0 with
+// multiple of 32, X and U_1 16-byte aligned): an SGEMM-style tile,
+// transposed.  A CTA owns RQ = 128 rows q of mode 0 with
 // their U_0 rows staged once in shared memory (rank-major), and walks a
 // contiguous range of RK = 32-column stages of the "rest" index; a stage's
 // 32 Khatri-Rao columns are 32 consecutive rows of U_1 times one constant
