@@ -225,13 +225,13 @@ __device__ __forceinline__ void load_u_item(const float *us, int r, int kc, floa
     u1 = *reinterpret_cast<const float4 *>(us + r * BKS + (((2 * kc + 1) ^ (r & 7)) << 2));
 }
 
-// Packs 16 consecutive contraction values x[k0..k0+15] of an A row into 8
-// hi words (and, for BF16x3, 8 lo words), two values per word.
-__device__ __forceinline__ void split_half(const float (&x)[BKS], int k0, uint32_t (&hi)[8], uint32_t (&lo)[8],
-                                           bool three, bool f16) {
+// Packs 16 consecutive contraction values of an A row into 8 hi words (and,
+// for BF16x3, 8 lo words), two values per word.
+__device__ __forceinline__ void split_half(const float *x, uint32_t (&hi)[8], uint32_t (&lo)[8], bool three,
+                                           bool f16) {
 #pragma unroll
     for (int c = 0; c < 8; c++) {
-        const float a0 = x[k0 + 2 * c], a1 = x[k0 + 2 * c + 1];
+        const float a0 = x[2 * c], a1 = x[2 * c + 1];
         lo[c] = 0u;
         if (f16) hi[c] = pack_f16(a0, a1);
         else if (three) split_pair(a0, a1, hi[c], lo[c]);
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(NTHREADS, MINB)
             // A stage: hi in columns 0-15, lo in 16-31 (2 values per column),
             // as two halves of 16 contraction values
             uint32_t hi0[8], lo0[8], hi1[8], lo1[8];
-            split_half(x, 0, hi0, lo0, three, f16);
-            split_half(x, 16, hi1, lo1, three, f16);
+            split_half(x, hi0, lo0, three, f16);
+            split_half(x + 16, hi1, lo1, three, f16);
             // A release must follow the instructions that consume the loaded
             // values: an arrive issued while a shared-memory load is still in
             // flight lets the next TMA overwrite the data under it.  The split
@@ -873,7 +873,13 @@ __global__ void __launch_bounds__(256) k_pack_b(KrFactors fold, long R, int Rpad
     *reinterpret_cast<uint4 *>(tile + bbytes + off) = l;
 }
 
-template <int MINB>
+// The precision (0: BF16, 1: three-term BF16, 2: FP16) and the kind of the
+// contraction are template arguments: as tests inside the converters' unrolled
+// loops they made 350 instructions a warp and stage, half of the SM's issue
+// slots.  With that, and X taken in halves of a stage (no spills at two CTAs an
+// SM), B200: 96^4 R = 32 79 -> 76 us a mode (BF16x3), 67 -> 60 (BF16); 512^3
+// R = 64 106 -> 104.
+template <int MINB, int kPrec, int kKind>
 __global__ void __launch_bounds__(PB_THREADS, MINB)
     k_mttkrp_pb(const __grid_constant__ CUtensorMap tmap, TcArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -926,23 +932,22 @@ __global__ void __launch_bounds__(PB_THREADS, MINB)
     ptx::tc_fence_after();
     const uint32_t tbase = sm.tmem_base;
 
-    const bool three = (a.prec == CUD_PREC_BF16X3 || a.prec == CUD_PREC_DEFAULT);
-    const bool f16 = (a.prec == CUD_PREC_FP16);
+    constexpr bool three = kPrec == 1, f16 = kPrec == 2;
 
     long issued_x = 0, issued_b = 0;  // copies issued (producer thread)
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
             Ring xr(nx), br(nb);
-            long ks = (a.kind == 0) ? 0 : st_beg / a.psteps;
-            long kp = (a.kind == 0) ? st_beg : st_beg % a.psteps;
+            long ks = (kKind == 0) ? 0 : st_beg / a.psteps;
+            long kp = (kKind == 0) ? st_beg : st_beg % a.psteps;
             long pos = st_beg % a.blk;  // stage position in its block = B tile
             bool packed = false;        // the pack kernel's tiles are visible
             for (long i = 0; i < nst && !*abort; i++) {
                 if (xr.use > 0 && !ptx::mbar_wait(&sm.empty_x[xr.slot], xr.prev_parity(), abort)) break;
                 uint8_t *dst = xring + (size_t)xr.slot * X_STAGE_BYTES;
                 ptx::mbar_arrive_expect_tx(&sm.full_x[xr.slot], (uint32_t)X_STAGE_BYTES);
-                if (a.kind == 0) ptx::tma_load_2d(dst, &tmap, &sm.full_x[xr.slot], (int)q0, (int)(kp * BKS));
+                if (kKind == 0) ptx::tma_load_2d(dst, &tmap, &sm.full_x[xr.slot], (int)q0, (int)(kp * BKS));
                 else ptx::tma_load_3d(dst, &tmap, &sm.full_x[xr.slot], (int)(kp * BKS), (int)q0, (int)ks);
                 issued_x = i + 1;
                 // the slot's B tile is free once the MMA of stage i - nb is done
@@ -958,7 +963,7 @@ __global__ void __launch_bounds__(PB_THREADS, MINB)
                 xr.next();
                 br.next();
                 kp++;
-                if (a.kind != 0 && kp == a.psteps) {
+                if (kKind != 0 && kp == a.psteps) {
                     kp = 0;
                     ks++;
                 }
@@ -1074,32 +1079,30 @@ __global__ void __launch_bounds__(PB_THREADS, MINB)
             if (use > 0 && !*abort) ptx::mbar_wait(&sm.empty_a[slot], (uint32_t)((use - 1) & 1), abort);
             if (!*abort) ptx::mbar_wait(&sm.full_x[xslot], (uint32_t)(xuse & 1), abort);
             __syncwarp();
-            float x[BKS];
             const float *xs = reinterpret_cast<const float *>(xring + (size_t)xslot * X_STAGE_BYTES);
-            if (a.kind == 0) {
+            const uint32_t ta = tbase + lane_off + a_col0 + (uint32_t)slot * 32u;
 #pragma unroll
-                for (int k = 0; k < BKS; k++) x[k] = xs[k * BQ + row];
-            } else {
-                const float4 *r4 = reinterpret_cast<const float4 *>(xs + row * BKS);
+            for (int half = 0; half < 2; half++) {
+                float x[16];
+                if (kKind == 0) {
 #pragma unroll
-                for (int c = 0; c < BKS / 4; c++) {
-                    float4 v = r4[c ^ (row & 7)];
-                    x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
+                    for (int k = 0; k < 16; k++) x[k] = xs[(16 * half + k) * BQ + row];
+                } else {
+                    const float4 *r4 = reinterpret_cast<const float4 *>(xs + row * BKS);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        const float4 v = r4[(4 * half + c) ^ (row & 7)];
+                        x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
+                    }
                 }
+                uint32_t hi[8], lo[8];
+                split_half(x, hi, lo, three, f16);
+                ptx::tmem_st8(ta + 8u * half, hi);
+                if (three) ptx::tmem_st8(ta + 16u + 8u * half, lo);
             }
-            uint32_t hi0[8], lo0[8], hi1[8], lo1[8];
-            split_half(x, 0, hi0, lo0, three, f16);
-            split_half(x, 16, hi1, lo1, three, f16);
             // released after the split, which reads every loaded X value
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&sm.empty_x[xslot]);
-            const uint32_t ta = tbase + lane_off + a_col0 + (uint32_t)slot * 32u;
-            ptx::tmem_st8(ta, hi0);
-            ptx::tmem_st8(ta + 8u, hi1);
-            if (three) {
-                ptx::tmem_st8(ta + 16u, lo0);
-                ptx::tmem_st8(ta + 24u, lo1);
-            }
             ptx::tmem_wait_st();
             ptx::tc_fence_before();
             __syncwarp();
@@ -1318,19 +1321,31 @@ int launch_tc(const CUtensorMap &tmap, const CUtensorMap &umap, const TcArgs &a,
     return CUD_OK;
 }
 
-template <int MINB>
-int launch_pb(const CUtensorMap &tmap, const TcArgs &a, size_t smem, unsigned grid, cudaStream_t s) {
+template <int MINB, int kPrec, int kKind>
+int launch_pb_as(const CUtensorMap &tmap, const TcArgs &a, size_t smem, unsigned grid, cudaStream_t s) {
     static std::atomic<bool> attr[64];  // per device; zero-initialised
     int dev = 0;
     CUD_CHECK(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !attr[dev].load(std::memory_order_acquire)) {
-        CUD_CHECK(cudaFuncSetAttribute(k_mttkrp_pb<MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+        CUD_CHECK(cudaFuncSetAttribute(k_mttkrp_pb<MINB, kPrec, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
         attr[dev].store(true, std::memory_order_release);
     }
     PdlLaunch l(grid, PB_THREADS, smem, s);  // overlaps the B pack (see griddep_wait)
-    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, k_mttkrp_pb<MINB>, tmap, a));
+    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, k_mttkrp_pb<MINB, kPrec, kKind>, tmap, a));
     CUD_CHECK_LAUNCH("mttkrp_pb");
     return CUD_OK;
+}
+
+template <int MINB>
+int launch_pb(const CUtensorMap &tmap, const TcArgs &a, size_t smem, unsigned grid, cudaStream_t s) {
+    const int prec = (a.prec == CUD_PREC_FP16) ? 2 : (a.prec == CUD_PREC_BF16) ? 0 : 1;
+    if (a.kind == 0)
+        return prec == 0   ? launch_pb_as<MINB, 0, 0>(tmap, a, smem, grid, s)
+               : prec == 1 ? launch_pb_as<MINB, 1, 0>(tmap, a, smem, grid, s)
+                           : launch_pb_as<MINB, 2, 0>(tmap, a, smem, grid, s);
+    return prec == 0   ? launch_pb_as<MINB, 0, 1>(tmap, a, smem, grid, s)
+           : prec == 1 ? launch_pb_as<MINB, 1, 1>(tmap, a, smem, grid, s)
+                       : launch_pb_as<MINB, 2, 1>(tmap, a, smem, grid, s);
 }
 
 }  // namespace
