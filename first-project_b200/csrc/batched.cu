@@ -21,9 +21,10 @@
 //     converged and skipped by later sweeps.
 // The host captures `sweeps_per_graph` sweeps (queue reset + kernel) in one
 // CUDA graph and replays it until every tensor has converged or hit the
-// sweep limit.  The CTA size and the CTAs per SM come from a small autotuner
-// (batched_tune) that times two sweeps per candidate on the batch itself and
-// caches the winner per batch shape class.
+// sweep limit.  The CTAs a tensor and per SM come from a rule on the number of
+// tensors (default_cfg), or from a small autotuner (cud_cp_batched_tune) that
+// times two sweeps per candidate on the batch itself and caches the winner per
+// batch shape class.
 #include <cooperative_groups.h>
 
 #include <atomic>
@@ -944,8 +945,8 @@ extern "C" int cud_cp_batched_tune(int ntensors, const long *dims, const long *r
         hr[t] = (int)ranks[t];
     }
     long key = shape_class(ntensors, hd.data(), hr.data());
-    // (threads, CTAs per SM) within the launch bounds' register budgets and
-    // shared memory (~45 KB a CTA)
+    // (threads, CTAs per SM, CTAs a tensor): two CTAs of 168 registers a thread
+    // and ~100 KB of shared memory fill an SM
     const std::vector<BatchCfg> cand = {{192, 2, 1}, {192, 2, 2}, {192, 2, 4}, {192, 2, 8}};
     BatchCfg bestc = default_cfg(ntensors);
     cudaStream_t s = as_stream(stream);

@@ -14,7 +14,7 @@
 // When the tiles alone cannot fill the GPU the contraction is split over
 // gridDim.z and a second kernel sums the FP32 partials in a fixed order and
 // applies the same epilogue.  Every wait is bounded (abort flag, drained
-// copies, TMEM freed); a CTA that gives up writes NaN.
+// copies, TMEM freed); a CTA that gives up takes NaN for its accumulators.
 //
 // All kernels here are launched programmatically (each waits for the one
 // before it ahead of its first global access, and lets the next start), so a

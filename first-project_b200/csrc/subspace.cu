@@ -258,7 +258,7 @@ constexpr size_t CL_SMEM_MAX = 200 * 1024;
 
 // Dynamic shared memory of the cluster kernels (offsets in doubles): two
 // row blocks (nl x 32, zero beyond column r), the two r x r buffers the
-// peers read, the 4 x 4 tile partials, two 32 x 32 matrices.
+// peers read, the tile partials, two 32 x 32 matrices.
 struct ClLayout {
     int nl;  // rows per CTA
     size_t ya, yb, red, gp, C, T, total;
