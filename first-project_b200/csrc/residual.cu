@@ -12,7 +12,10 @@
 // forms 2 x 8 reconstructed entries xh = sum_r U_0[i, r] W[r][j] in FP32 and
 // accumulates (x - xh)^2 and x^2 in FP64.  X is read once, coalesced
 // along mode 0.  Per-CTA partials are summed in a fixed order by a second
-// kernel, so the result is deterministic.
+// kernel, so the result is deterministic.  A pass runs over the ranks it
+// has, in fours (its bound is the shared memory that feeds the FMAs: B200, 253 x
+// 211 x 187 at R = 20 82 -> 54 us, 130 x 70 x 50 x 30 at R = 8 176 -> 96, against
+// passes padded to 64 ranks and 64-bit digits; at R = 64 99 -> 95).
 //
 // Shapes that allow it take an FFMA-tiled fast path (k_residual_ffma below).
 //
@@ -64,9 +67,11 @@ __global__ void __launch_bounds__(NT) k_cp_residual(ResArgs a) {
     const int wj = threadIdx.x % TJ, wg = threadIdx.x / TJ;
     const long nchunks = (a.rest + TJ - 1) / TJ;
     const bool one_pass = a.R <= RC;  // U_0's tile fits: load it once
+    const bool small = a.rest <= 0x7fffffffL;  // then every chunk's last index fits 32 bits too
     double acc = 0.0, xx = 0.0;
+    const auto ranks = [&](long rc) { return ((int)min((long)RC, a.R - rc) + 3) & ~3; };  // of a pass, in fours
     if (one_pass) {
-        for (int e = threadIdx.x; e < RC * TI; e += NT) {
+        for (int e = threadIdx.x; e < ranks(0) * TI; e += NT) {
             const int r = e / TI, t = e % TI;
             const long i = blockIdx.x * (long)TI + t;
             U0s[r][t] = (r < a.R && i < a.I0) ? a.U0[i + a.I0 * r] : 0.f;
@@ -89,6 +94,8 @@ __global__ void __launch_bounds__(NT) k_cp_residual(ResArgs a) {
         long ws[kMaxOrder];
         const bool wok = rest0 + wj < a.rest;
         {
+            // (32-bit digits where the rest index fits: a 64-bit division takes
+            // some hundred clocks)
             long lin = rest0 + wj;
 #pragma unroll
             for (int m = 0; m < kMaxOrder; m++) {
@@ -96,16 +103,18 @@ __global__ void __launch_bounds__(NT) k_cp_residual(ResArgs a) {
                 ws[m] = 0;
                 if (m < nf) {
                     const long d = fRows[m];
-                    wb[m] = fU[m] + (lin % d);
+                    const long q = small ? (long)((unsigned)lin / (unsigned)d) : lin / d;
+                    wb[m] = fU[m] + (lin - q * d);
                     ws[m] = d;
-                    lin /= d;
+                    lin = q;
                 }
             }
         }
         for (long rc = 0; rc < a.R; rc += RC) {
+            const int rn = ranks(rc);
             __syncthreads();
             if (!one_pass) {
-                for (int e = threadIdx.x; e < RC * TI; e += NT) {
+                for (int e = threadIdx.x; e < rn * TI; e += NT) {
                     const int r = e / TI, t = e % TI;
                     const long i = blockIdx.x * (long)TI + t;
                     U0s[r][t] = (rc + r < a.R && i < a.I0) ? a.U0[i + a.I0 * (rc + r)] : 0.f;
@@ -113,6 +122,7 @@ __global__ void __launch_bounds__(NT) k_cp_residual(ResArgs a) {
             }
 #pragma unroll
             for (int t = 0; t < RC / 8; t++) {
+                if (8 * t >= rn) break;
                 const int r = wg + 8 * t;
                 const long rr = rc + r;
                 float w = 0.f;
@@ -126,7 +136,7 @@ __global__ void __launch_bounds__(NT) k_cp_residual(ResArgs a) {
             }
             __syncthreads();
 #pragma unroll 4
-            for (int r = 0; r < RC; r++) {
+            for (int r = 0; r < rn; r++) {
                 const float u0 = U0s[r][ti], u1 = U0s[r][ti + 64];
                 const float4 w0 = *reinterpret_cast<const float4 *>(&Ws[r][rl * 8]);
                 const float4 w1 = *reinterpret_cast<const float4 *>(&Ws[r][rl * 8 + 4]);
