@@ -59,6 +59,16 @@ constexpr int RT_XJ = 32;       // U_1 rows (X columns) per X tile
 // bound by its per-slice chain (A' build -> MMA -> epilogue), not by the
 // bytes in flight.
 constexpr int RT_XSMAX = 12;
+// An epilogue warp waits for its own tile of each chunk only, so it does not
+// see every use of a ring slot, and a wait for a phase's parity also passes
+// while the use before the one meant is still on its way.  That tile, xs
+// before the warp's own, has landed for certain where it belongs to a chunk
+// whose accumulator every epilogue warp has released, i.e. two chunks back or
+// earlier: with a ring of two chunks' tiles.  In a shorter ring the warps
+// first wait until their tile's load has been issued (RtCtrl::issued), which
+// follows the release of the use before.  (B200, a call at 512^3 R = 64, ring
+// of 6: 164 us with this wait.)
+constexpr int RT_XSFREE = 2 * (RT_NJ / RT_XJ);
 constexpr int RT_THREADS = 832; // warp 0 TMA, 1 MMA, 2-9 builders, 10-25 epilogue
 constexpr int RT_BLD = 8;       // builder warps: two per TMEM lane quarter, 32 ranks each
 constexpr int RT_EPI = 16;      // epilogue warps: four per TMEM lane quarter, an X tile of a chunk each
@@ -83,6 +93,7 @@ struct RtCtrl {
     uint64_t a_full[2], a_free[2], d_full[2], d_free[2], done;
     uint32_t tmem_base;
     int abort;
+    uint32_t issued;  // X tiles whose loads have been issued
     const float *fU[kMaxOrder];
     long frows[kMaxOrder];
     float cvec[RT_BLD][32];
@@ -133,6 +144,17 @@ struct RtRing {
     }
 };
 
+// Waits (bounded, as mbar_wait) until the load of X tile `tile` is issued.
+__device__ __forceinline__ void rt_wait_issued(const uint32_t *issued, uint32_t tile, volatile int *abort) {
+    for (long i = 0; !*abort; i++) {
+        uint32_t n;
+        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(n) : "r"(ptx::smem_addr(issued)) : "memory");
+        if ((int)(n - tile) > 0) return;
+        __nanosleep(20);
+        if (i > (1L << 26)) *abort = 1;
+    }
+}
+
 __global__ void __launch_bounds__(RT_THREADS, 1)
     k_residual_tc(const __grid_constant__ CUtensorMap tmap, RtArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -162,6 +184,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
         }
         ptx::mbar_init(&sm.done, 1);
         sm.abort = 0;
+        sm.issued = 0;
 #pragma unroll
         for (int m = 0; m < kMaxOrder; m++) {  // constant indices: no local copy of the parameter
             sm.fU[m] = m < a.f.n ? a.f.U[m] : nullptr;
@@ -180,6 +203,9 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
         ptx::tma_load_3d(xring + (size_t)xl.slot * RT_XBYTES, &tmap, &sm.x_full[xl.slot], (int)i0,
                          xt * RT_XJ, (int)(k_beg + xk));
         issued_x++;
+        asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(ptx::smem_addr(&sm.issued)),
+                     "r"((uint32_t)issued_x)
+                     : "memory");
         xl.next();
         if (++xt == ntiles) {
             xt = 0;
@@ -328,12 +354,15 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
         double sr[4] = {0.0, 0.0, 0.0, 0.0}, sx[4] = {0.0, 0.0, 0.0, 0.0};
         RtRing xr(a.xs);
         xr.next(g);
+        const bool short_ring = a.xs < RT_XSFREE;
+        uint32_t xi = (uint32_t)g;  // number of this warp's tile
         int q = 0;
         for (long ci = 0; ci < nchunks && !*abort; ci++) {
             const int db = (int)(ci & 1);
             const int tiles = min(RT_NJ / RT_XJ, ntiles - q * (RT_NJ / RT_XJ));  // X tiles of the chunk
             const bool mine = g < tiles;
             if (!*abort) ptx::mbar_wait(&sm.d_full[db], (uint32_t)((ci >> 1) & 1), abort);
+            if (mine && short_ring) rt_wait_issued(&sm.issued, xi, abort);
             if (mine && !*abort) ptx::mbar_wait(&sm.x_full[xr.slot], (uint32_t)(xr.use & 1), abort);
             const bool ok = __all_sync(0xffffffffu, *abort == 0);  // warp-uniform exit before tcgen05.ld
             if (!ok) break;
@@ -369,6 +398,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
                 ptx::mbar_arrive(&sm.d_free[db]);
             }
             xr.next(tiles);
+            xi += (uint32_t)tiles;
             if (++q == a.nq) q = 0;
         }
         s_res = (sr[0] + sr[1]) + (sr[2] + sr[3]);
