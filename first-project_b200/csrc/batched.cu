@@ -534,8 +534,11 @@ __global__ void __launch_bounds__(NW * 32, 2) k_batch_sweep(BatchArgs a) {
     uint32_t mails = 0;  // mails that this warp has waited for
     if (CL > 1 && threadIdx.x < NW) {
         ptx::mbar_init(&sm.mail_full[threadIdx.x], 1);
-        ptx::fence_mbar_init();  // (the cluster synchronises before the first mail)
+        ptx::fence_mbar_init();
     }
+    // every CTA of the cluster runs, and its barriers are set up, before a peer
+    // writes to its shared memory
+    if (CL > 1) cl.sync();
     for (;;) {
         if (rank == 0 && threadIdx.x == 0) {
             const unsigned w = atomicAdd(a.queue, 1u);
