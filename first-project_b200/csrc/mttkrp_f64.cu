@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(DT, DTile<kQ, NT>::MINB) k_mttkrp_f64(const __
     const int nrow = qleft <= 0 ? 0 : kQ == 0 ? NC : (int)min((long)NC, (qleft + STEP - 1) / STEP);
     const uint32_t xdst = smem_u32(Xring) + 8u * (kQ == 0 ? ck * LDQ + cq : cq * LDK + ck);
     constexpr uint32_t dstride = 8u * STEP * (kQ == 0 ? LDQ : LDK);
-    // U0: 16 lanes = rows, half-warps take the ranks in turn; ranks past R
+    // U0: 16 lanes = rows (those past the block's end are left as they are),
+    // half-warps take the ranks in turn; ranks past R
     // repeat rank R - 1 (their results are not written)
     const int bk = t % DK, bc = t / DK;
     const uint32_t bdst = smem_u32(Bring) + 8u * (bk * T::LDB + bc);
@@ -149,7 +150,6 @@ __global__ void __launch_bounds__(DT, DTile<kQ, NT>::MINB) k_mttkrp_f64(const __
         for (int i = 0; i < NT; i++) {
             const I r = (I)min(r0 + bc + 8 * i, a.R - 1);
             if (bk < kc) copy_async<8>(bd + 64u * i, a.U[0] + (row + r * (I)rows0));
-            else zero8(bd + 64u * i);
         }
         // the next stage
         lj++;
@@ -207,12 +207,16 @@ __global__ void __launch_bounds__(DT, DTile<kQ, NT>::MINB) k_mttkrp_f64(const __
         const int fr = 32 * warp + (lane >> 2), fk = lane & 3;
         const double *A = Xring + slot * AF + (kQ == 0 ? fk * LDQ + fr : fr * LDK + fk);
         const double *B = Bring + slot * BF + fk * T::LDB + (lane >> 2);
-        auto step = [&](int k) {
+        // `in`: this lane's kappa is in the block.  Past its end X is zero, and
+        // the Khatri-Rao value is too, not a product that an infinite constant
+        // row would turn into NaN.  (B200, 253 x 211 x 187 R = 20: 29 / 34 / 38 us
+        // a mode without this, 29 / 36 / 40 with it.)
+        auto step = [&](int k, bool in) {
             double x[MT], y[NT];
 #pragma unroll
             for (int m = 0; m < MT; m++) x[m] = A[kQ == 0 ? k * LDQ + 8 * m : 8 * m * LDK + k];
 #pragma unroll
-            for (int j = 0; j < NT; j++) y[j] = B[k * T::LDB + 8 * j] * cc[j];
+            for (int j = 0; j < NT; j++) y[j] = in ? B[k * T::LDB + 8 * j] * cc[j] : 0.0;
 #pragma unroll
             for (int m = 0; m < MT; m++)
 #pragma unroll
@@ -220,10 +224,12 @@ __global__ void __launch_bounds__(DT, DTile<kQ, NT>::MINB) k_mttkrp_f64(const __
         };
         if (kc == DK) {
 #pragma unroll
-            for (int k = 0; k < DK; k += 4) step(k);
+            for (int k = 0; k < DK; k += 4) step(k, true);
         } else {
+            int k = 0;
 #pragma unroll 1
-            for (int k = 0; k < kc; k += 4) step(k);
+            for (; k + 4 <= kc; k += 4) step(k, true);
+            if (k < kc) step(k, k + fk < kc);
         }
         slot = slot + 1 == DST ? 0 : slot + 1;
         if (++cj == bsteps) {
