@@ -56,7 +56,9 @@ constexpr size_t GCTRL_BYTES = 1024;
 __host__ __device__ constexpr size_t gemm_stage_bytes(int BN) { return (size_t)(GBM + BN) * GBK * 2; }
 __host__ __device__ constexpr size_t gemm_smem_bytes(int BN) { return 1024 + GCTRL_BYTES + GST * gemm_stage_bytes(BN); }
 
-// The fused epilogue for one element (m, n) with accumulator value v.
+// The fused epilogue for one element (m, n) with accumulator value v.  A NaN
+// (also that of a CTA that gave up) passes the ReLU; an element that the mask
+// takes out is zero whatever its sum.
 __device__ __forceinline__ void epi_store(const GemmEpi &e, long m, long n, float v) {
     v *= e.alpha;
     if (e.bias) v += e.bias[n];
@@ -64,7 +66,7 @@ __device__ __forceinline__ void epi_store(const GemmEpi &e, long m, long n, floa
         const __nv_bfloat16 *mk = static_cast<const __nv_bfloat16 *>(e.mask);
         if (!(__bfloat162float(mk[m * e.mask_ldm + n * e.mask_ldn]) > 0.f)) v = 0.f;
     }
-    if (e.relu) v = fmaxf(v, 0.f);
+    if (e.relu && !(v > 0.f) && v == v) v = 0.f;
     if (e.out_f32) {
         float *p = e.out_f32 + m * e.f32_ldm + n * e.f32_ldn;
         *p = e.f32_accumulate ? *p + v : v;
