@@ -17,9 +17,12 @@
 // copies, TMEM freed); a CTA that gives up takes NaN for its accumulators.
 //
 // All kernels here are launched programmatically (each waits for the one
-// before it ahead of its first global access, and lets the next start), so a
-// chain of products does not pay a launch gap between them (B200, HOSVD of a
-// 256^3 tensor at rank 16, 12 products: 782 -> 735 us).
+// before it ahead of its first global access), so a chain of products does not
+// pay a launch gap between them (B200, HOSVD of a 256^3 tensor at rank 16, 12
+// products: 782 -> 730 us).  The skinny product and the split sum also let the
+// next kernel start; k_gemm_tc does not, since its dependents' CTAs took more
+// from its last wave than their early start gave (8192 x 8192 x 64 525
+// against 516 us, 1024^3 32.2 against 27.9, the HOSVD 739 against 730).
 #include <atomic>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -66,7 +69,7 @@ __device__ __forceinline__ void epi_store(const GemmEpi &e, long m, long n, floa
         const __nv_bfloat16 *mk = static_cast<const __nv_bfloat16 *>(e.mask);
         if (!(__bfloat162float(mk[m * e.mask_ldm + n * e.mask_ldn]) > 0.f)) v = 0.f;
     }
-    if (e.relu && !(v > 0.f) && v == v) v = 0.f;
+    if (e.relu) asm("max.NaN.f32 %0, %0, %1;" : "+f"(v) : "f"(0.f));
     if (e.out_f32) {
         float *p = e.out_f32 + m * e.f32_ldm + n * e.f32_ldn;
         *p = e.f32_accumulate ? *p + v : v;
@@ -114,7 +117,6 @@ __global__ void __launch_bounds__(GTHREADS, 1)
     const uint32_t tbase = sm.tmem_base;
     // launched programmatically: everything above overlaps the kernel before
     ptx::griddep_wait();
-    ptx::griddep_launch();
 
     long issued = 0;
     if (warp == 0) {
@@ -159,17 +161,12 @@ __global__ void __launch_bounds__(GTHREADS, 1)
         bool ok = true;
         if (!*abort) ok = ptx::mbar_wait(&sm.done, 0u, abort);
         ok = __all_sync(0xffffffffu, ok && *abort == 0 && nkb > 0);
-        {
-            if (ok) ptx::tc_fence_after();
+        if (ok) {
+            ptx::tc_fence_after();
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t v[32];
-                if (ok) {
-                    ptx::tmem_ld32(tbase + lane_off + (uint32_t)c0, v);
-                    ptx::tmem_wait_ld();
-                } else {  // gave up: the result must not pass for a value
-#pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] = 0x7fffffffu;
-                }
+                ptx::tmem_ld32(tbase + lane_off + (uint32_t)c0, v);
+                ptx::tmem_wait_ld();
                 if (m < g.M) {
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
@@ -182,7 +179,15 @@ __global__ void __launch_bounds__(GTHREADS, 1)
                     }
                 }
             }
-            if (ok) ptx::tc_fence_before();
+            ptx::tc_fence_before();
+        } else if (m < g.M) {  // gave up: the result must not pass for a value
+            const float val = __uint_as_float(0x7fffffffu);
+            const long n1 = min(g.N, n0 + BN);
+#pragma unroll 1
+            for (long n = n0; n < n1; n++) {
+                if (g.part) g.part[((long)blockIdx.z * g.N + n) * g.M + m] = val;
+                else epi_store(g.e, m, n, val);
+            }
         }
     }
 
