@@ -62,12 +62,10 @@ int round_mode(int precision) {
 
 int sum_splits(const float *part, int splits, long Q, long R, long Rp, const int *error, float *out, cudaStream_t s) {
     const long ctas = (Q * (Rp ? Rp : R) + 31) / 32;
-    // 32 lanes an output where the splits feed them and the grid is about a
-    // wave of such CTAs (B200, a call: 96^4 R = 32, 294 splits of 96 CTAs 4.4
-    // against 8.1 us; 512^3 R = 64, 73 splits of 1024 CTAs 10.6 against 5.0)
-    const bool wide = splits >= 32 && ctas <= 4L * kNumSMs;
-    PdlLaunch l((unsigned)ctas, wide ? 1024 : 256, 0, s);
-    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, wide ? k_sum_splits<32> : k_sum_splits<8>, part, splits, Q, R, Rp, error, out));
+    const int lanes = sum_lanes(splits, ctas);
+    PdlLaunch l((unsigned)ctas, 32 * lanes, 0, s);
+    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, lanes == 32 ? k_sum_splits<32> : lanes == 8 ? k_sum_splits<8> : k_sum_splits<1>,
+                                 part, splits, Q, R, Rp, error, out));
     CUD_CHECK_LAUNCH("mttkrp reduce");
     return CUD_OK;
 }

@@ -256,8 +256,8 @@ __global__ void __launch_bounds__(DT, DTile<kQ, NT>::MINB) k_mttkrp_f64(const __
 }
 
 // out[e] = sum_z part[z][e]: a CTA owns 32 consecutive outputs, ZL lanes each
-// over the splits, then a fixed two-level order.
-constexpr int ZL = 32;
+// over the splits, then a fixed order (two levels for 32 lanes).
+template <int ZL>
 __global__ void __launch_bounds__(32 * ZL) k_sum_splits_f64(const double *__restrict__ part, int splits, long n,
                                                             double *__restrict__ out) {
     __shared__ double red[ZL][32];
@@ -271,13 +271,18 @@ __global__ void __launch_bounds__(32 * ZL) k_sum_splits_f64(const double *__rest
     }
     red[zl][o] = sum;
     __syncthreads();
-    if (zl < 4) {
+    constexpr int G = ZL > 8 ? 4 : 1;  // second-level sums
+    if (zl < G) {
 #pragma unroll
-        for (int k = zl + 4; k < ZL; k += 4) sum += red[k][o];
-        red[zl][o] = sum;
+        for (int k = zl + G; k < ZL; k += G) sum += red[k][o];
+        if (G > 1) red[zl][o] = sum;
     }
-    __syncthreads();
-    if (zl == 0 && e < n) out[e] = sum + red[1][o] + red[2][o] + red[3][o];
+    if (G > 1) __syncthreads();
+    if (zl == 0 && e < n) {
+#pragma unroll
+        for (int k = 1; k < G; k++) sum += red[k][o];
+        out[e] = sum;
+    }
 }
 
 struct F64Plan {
@@ -376,8 +381,11 @@ int mttkrp_f64(const double *X, int order, const long *dims, const double *const
     prof_end(pk, s);
     if (st) return st;
     const long n = R * v.Q;
-    PdlLaunch l((unsigned)((n + 31) / 32), 32 * ZL, 0, s);
-    CUD_CHECK(cudaLaunchKernelEx(&l.cfg, k_sum_splits_f64, (const double *)a.part, (int)p.splits, n, out));
+    const int lanes = sum_lanes((int)p.splits, (n + 31) / 32);
+    PdlLaunch l((unsigned)((n + 31) / 32), 32 * lanes, 0, s);
+    CUD_CHECK(cudaLaunchKernelEx(
+        &l.cfg, lanes == 32 ? k_sum_splits_f64<32> : lanes == 8 ? k_sum_splits_f64<8> : k_sum_splits_f64<1>,
+        (const double *)a.part, (int)p.splits, n, out));
     CUD_CHECK_LAUNCH("mttkrp_f64 reduce");
     return CUD_OK;
 }
