@@ -117,16 +117,17 @@ struct MttkrpParts {
 // layout is returned there and `out` is not written.
 int mttkrp_tc(const float *X, int order, const long *dims, const float *const *U, int mode,
               long R, float *out, int precision, void *ws, cudaStream_t s, MttkrpParts *parts = nullptr);
-// Lanes per output of a split reduce over `ctas` groups of 32 outputs: 32
-// where the splits feed them and the grid is within a wave of such CTAs (B200,
-// a call: 96^4 R = 32, 294 splits of 96 CTAs 4.4 against 8.1 us; 512^3 R = 64, 73
-// splits of 1024 CTAs 10.6 against 5.0; with the MTTKRP, 160^3 R = 64, 320 CTAs,
-// 22.6 against 20.8), one where there are fewer splits than lanes (with the
-// MTTKRP, FP64 100000 x 6 x 6 R = 8, one split of 25000 CTAs, 78 us with 32
-// lanes, 28 with one; FP32 32 with 8, 28 with one).
-inline int sum_lanes(int splits, long ctas) {
-    return splits >= 32 && ctas < 2L * kNumSMs ? 32 : splits >= 8 ? 8 : 1;
+// Lanes per output of a split reduce over n outputs: 32 where the splits feed
+// them and the grid is within a wave of such CTAs (B200, a call: 96^4 R = 32, 294
+// splits of 96 CTAs 4.4 against 8.1 us; 512^3 R = 64, 73 splits of 1024 CTAs 10.6
+// against 5.0; with the MTTKRP, 160^3 R = 64, 320 CTAs, 22.6 against 20.8), one
+// where there are fewer splits than lanes.  And outputs per CTA: 32, or 256 of
+// one lane each (with the MTTKRP, 100000 x 6 x 6 R = 8, one split: FP64 18 us, 28
+// with 32 outputs a CTA, 78 with 32 lanes; FP32 17, 32 with 8 lanes).
+inline int sum_lanes(int splits, long n) {
+    return splits >= 32 && (n + 31) / 32 < 2L * kNumSMs ? 32 : splits >= 8 ? 8 : 1;
 }
+__host__ __device__ constexpr int sum_width(int lanes) { return lanes == 1 ? 256 : 32; }
 // The split reduce (mttkrp.cu): out (Q x R, column-major) = the sum of the
 // partials over the splits in FP64, in a fixed order.  Rp = 0: partials
 // [split][r][q]; else [split][q][Rp].  NaN everywhere when *error is set.

@@ -14,17 +14,18 @@ namespace cud {
 
 namespace {
 
-// A CTA owns 32 consecutive slots of a partial (coalesced reads), each summed
-// by ZL lanes over the splits z = lane, lane + ZL, .. and then in a fixed
+// A CTA owns OW (32, or 256 for one lane each) consecutive slots of a partial
+// (coalesced reads), each summed by ZL lanes over the splits z = lane, lane + ZL, .. and then in a fixed
 // two-level order.  Bound: the latency of the chain of L2 reads, so the lanes
 // are as many as the splits can feed.
 template <int ZL>
-__global__ void __launch_bounds__(32 * ZL) k_sum_splits(const float *__restrict__ part, int splits, long Q, long R,
+__global__ void __launch_bounds__(sum_width(ZL) * ZL) k_sum_splits(const float *__restrict__ part, int splits, long Q, long R,
                                                         long Rp, const int *__restrict__ error,
                                                         float *__restrict__ out) {
-    __shared__ double red[ZL][32];
-    const int o = threadIdx.x & 31, zl = threadIdx.x >> 5;
-    const long e = blockIdx.x * 32L + o;
+    constexpr int OW = sum_width(ZL);
+    __shared__ double red[ZL][OW];
+    const int o = threadIdx.x % OW, zl = threadIdx.x / OW;
+    const long e = blockIdx.x * (long)OW + o;
     const long n = Q * (Rp ? Rp : R);
     ptx::griddep_wait();  // the partials
     double sum = 0.0;
@@ -61,9 +62,9 @@ int round_mode(int precision) {
 }  // namespace
 
 int sum_splits(const float *part, int splits, long Q, long R, long Rp, const int *error, float *out, cudaStream_t s) {
-    const long ctas = (Q * (Rp ? Rp : R) + 31) / 32;
-    const int lanes = sum_lanes(splits, ctas);
-    PdlLaunch l((unsigned)ctas, 32 * lanes, 0, s);
+    const long n = Q * (Rp ? Rp : R);
+    const int lanes = sum_lanes(splits, n), ow = sum_width(lanes);
+    PdlLaunch l((unsigned)((n + ow - 1) / ow), ow * lanes, 0, s);
     CUD_CHECK(cudaLaunchKernelEx(&l.cfg, lanes == 32 ? k_sum_splits<32> : lanes == 8 ? k_sum_splits<8> : k_sum_splits<1>,
                                  part, splits, Q, R, Rp, error, out));
     CUD_CHECK_LAUNCH("mttkrp reduce");

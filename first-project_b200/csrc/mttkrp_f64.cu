@@ -255,14 +255,15 @@ __global__ void __launch_bounds__(DT, DTile<kQ, NT>::MINB) k_mttkrp_f64(const __
     ptx::griddep_launch();
 }
 
-// out[e] = sum_z part[z][e]: a CTA owns 32 consecutive outputs, ZL lanes each
-// over the splits, then a fixed order (two levels for 32 lanes).
+// out[e] = sum_z part[z][e]: a CTA owns sum_width(ZL) consecutive outputs, ZL
+// lanes each over the splits, then a fixed order (two levels for 32 lanes).
 template <int ZL>
-__global__ void __launch_bounds__(32 * ZL) k_sum_splits_f64(const double *__restrict__ part, int splits, long n,
+__global__ void __launch_bounds__(sum_width(ZL) * ZL) k_sum_splits_f64(const double *__restrict__ part, int splits, long n,
                                                             double *__restrict__ out) {
-    __shared__ double red[ZL][32];
-    const int o = threadIdx.x & 31, zl = threadIdx.x >> 5;
-    const long e = blockIdx.x * 32L + o;
+    constexpr int OW = sum_width(ZL);
+    __shared__ double red[ZL][OW];
+    const int o = threadIdx.x % OW, zl = threadIdx.x / OW;
+    const long e = blockIdx.x * (long)OW + o;
     ptx::griddep_wait();  // the partials
     double sum = 0.0;
     if (e < n) {
@@ -381,8 +382,8 @@ int mttkrp_f64(const double *X, int order, const long *dims, const double *const
     prof_end(pk, s);
     if (st) return st;
     const long n = R * v.Q;
-    const int lanes = sum_lanes((int)p.splits, (n + 31) / 32);
-    PdlLaunch l((unsigned)((n + 31) / 32), 32 * lanes, 0, s);
+    const int lanes = sum_lanes((int)p.splits, n), ow = sum_width(lanes);
+    PdlLaunch l((unsigned)((n + ow - 1) / ow), ow * lanes, 0, s);
     CUD_CHECK(cudaLaunchKernelEx(
         &l.cfg, lanes == 32 ? k_sum_splits_f64<32> : lanes == 8 ? k_sum_splits_f64<8> : k_sum_splits_f64<1>,
         (const double *)a.part, (int)p.splits, n, out));
