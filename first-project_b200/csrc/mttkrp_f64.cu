@@ -1,8 +1,8 @@
 // MTTKRP on FP64 data (the FP64 CP-ALS), any order and extents, in the
 // tensor's native layout, with no Khatri-Rao matrix:
 //     M[q, r] = sum_kappa X(q, kappa) KR(kappa, r),
-// kappa = s for mode 0 (q contiguous in memory), kappa = p + P s for the
-// other modes (p contiguous).
+// kappa = s where P = 1 (mode 0; q contiguous in memory), kappa = p + P s for
+// the other modes (p contiguous).
 //
 // Bound: HBM up to rank ~20 (2 R flops for 8 bytes against 37 TFLOP/s and
 // 6.5 TB/s), FP64 arithmetic above.  The multiply-adds are the FP64 matrix
@@ -297,7 +297,8 @@ struct F64Plan {
 F64Plan f64_plan(int order, const long *dims, int mode, long R) {
     const ModeView v = mode_view(order, dims, mode);
     F64Plan p;
-    const long rows0 = dims[mode == 0 ? 1 : 0], blocks = v.P * v.S / rows0;
+    int oth[kMaxOrder];
+    const long rows0 = other_modes(order, dims, mode, oth) ? dims[oth[0]] : 1, blocks = v.P * v.S / rows0;
     p.bsteps = (rows0 + DK - 1) / DK;
     p.steps = blocks * p.bsteps;
     p.any = blocks > 0x3fffffffL || p.steps > 0x7fffffffL;
@@ -358,14 +359,15 @@ int mttkrp_f64(const double *X, int order, const long *dims, const double *const
     a.X = X;
     a.P = v.P; a.Q = v.Q; a.S = v.S;
     a.R = (int)R;
-    a.nf = 0;
-    for (int m = 0; m < order; m++) {
-        if (m == mode) continue;
-        a.U[a.nf] = U[m];
-        a.rows[a.nf++] = dims[m];
+    int oth[kMaxOrder];
+    a.nf = other_modes(order, dims, mode, oth);
+    for (int f = 0; f < a.nf; f++) {
+        a.U[f] = U[oth[f]];
+        a.rows[f] = dims[oth[f]];
     }
     a.bsteps = p.bsteps;
-    a.pblocks = mode == 0 ? 1 : v.P / a.rows[0];
+    const bool qfast = v.P == 1;  // q is contiguous in memory
+    a.pblocks = qfast ? 1 : v.P / a.rows[0];
     a.qtiles = p.qtiles;
     a.steps = p.steps;
     a.chunk = p.chunk;
@@ -373,11 +375,11 @@ int mttkrp_f64(const double *X, int order, const long *dims, const double *const
     const dim3 grid((unsigned)(p.qtiles * p.splits), (unsigned)p.rtiles);
     // 16-byte copies: whole ones along q, or of a row block of U0 (a pair that
     // crossed its end would multiply the next block's value by zero)
-    const bool vec = (mode == 0 ? v.Q : dims[0]) % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    const bool vec = (qfast ? v.Q : a.rows[0]) % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     const int pk = prof_begin(s);
     int st;
-    if (p.any) st = mode == 0 ? launch<0, false, true, 8>(a, grid, s) : launch<1, false, true, 8>(a, grid, s);
-    else if (mode == 0) st = vec ? launch_nt<0, true>(p, a, grid, s) : launch_nt<0, false>(p, a, grid, s);
+    if (p.any) st = qfast ? launch<0, false, true, 8>(a, grid, s) : launch<1, false, true, 8>(a, grid, s);
+    else if (qfast) st = vec ? launch_nt<0, true>(p, a, grid, s) : launch_nt<0, false>(p, a, grid, s);
     else st = vec ? launch_nt<1, true>(p, a, grid, s) : launch_nt<1, false>(p, a, grid, s);
     prof_end(pk, s);
     if (st) return st;

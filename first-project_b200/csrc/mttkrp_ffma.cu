@@ -4,8 +4,8 @@
 //
 // Around mode n the tensor is a (P, Q, S) array and
 //     M[q, r] = sum_kappa X(q, kappa) KR(kappa, r),
-// kappa = s for mode 0 (q contiguous in memory), kappa = p + P s for the other
-// modes (p contiguous), KR(kappa, r) the product of the other factors' rows at
+// kappa = s where P = 1 (mode 0; q contiguous in memory), kappa = p + P s for the
+// other modes (p contiguous), KR(kappa, r) the product of the other factors' rows at
 // kappa's digits.  X is read in its native layout, the Khatri-Rao rows are
 // formed per stage in shared memory, nothing is materialised.
 //
@@ -452,7 +452,8 @@ struct FfmaPlan {
 FfmaPlan ffma_plan(int order, const long *dims, int mode, long R, int round) {
     const ModeView v = mode_view(order, dims, mode);
     FfmaPlan p;
-    const long rows0 = dims[mode == 0 ? 1 : 0], blocks = v.P * v.S / rows0;
+    int oth[kMaxOrder];
+    const long rows0 = other_modes(order, dims, mode, oth) ? dims[oth[0]] : 1, blocks = v.P * v.S / rows0;
     p.any = round != 0 || blocks > 0x3fffffffL || blocks * ((rows0 + FK - 1) / FK) > 0x7fffffffL;
     for (int m = 0; m < order; m++) p.any = p.any || R * dims[m] > 0x3fffffffL;
     p.rtiles = (R + 63) / 64;
@@ -527,14 +528,15 @@ int mttkrp_ffma(const float *X, int order, const long *dims, const float *const 
     a.P = v.P; a.Q = v.Q; a.S = v.S;
     a.R = (int)R;
     a.round = round;
-    a.nf = 0;
-    for (int m = 0; m < order; m++) {
-        if (m == mode) continue;
-        a.U[a.nf] = U[m];
-        a.rows[a.nf++] = dims[m];
+    int oth[kMaxOrder];
+    a.nf = other_modes(order, dims, mode, oth);
+    for (int f = 0; f < a.nf; f++) {
+        a.U[f] = U[oth[f]];
+        a.rows[f] = dims[oth[f]];
     }
     a.bsteps = p.bsteps;
-    a.pblocks = mode == 0 ? 1 : v.P / a.rows[0];
+    const bool qfast = v.P == 1;  // q is contiguous in memory
+    a.pblocks = qfast ? 1 : v.P / a.rows[0];
     a.qtiles = p.qtiles;
     a.steps = p.steps;
     a.chunk = p.chunk;
@@ -544,9 +546,9 @@ int mttkrp_ffma(const float *X, int order, const long *dims, const float *const 
     // 16-byte copies: along q whole ones; along kappa also whole ones of a row
     // block of U0 (a group of 4 that crossed its end would multiply the next
     // block's values, which may be infinite, by zeros)
-    const bool vec = (mode == 0 ? v.Q : dims[0]) % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    const bool vec = (qfast ? v.Q : a.rows[0]) % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     const bool any = p.any;
-    const int st = mode == 0 ? (any ? launch_nr<0, false, true>(p, a, grid, s)
+    const int st = qfast ? (any ? launch_nr<0, false, true>(p, a, grid, s)
                                 : vec ? launch_nr<0, true, false>(p, a, grid, s) : launch_nr<0, false, false>(p, a, grid, s))
                              : (any ? launch_nr<2, false, true>(p, a, grid, s)
                                 : vec ? launch_nr<1, true, false>(p, a, grid, s) : launch_nr<2, false, false>(p, a, grid, s));
