@@ -103,6 +103,9 @@ inline int other_modes(int order, const long *dims, int mode, int (&out)[kMaxOrd
 size_t mttkrp_ffma_ws_bytes(int order, const long *dims, int mode, long R, int round);
 int mttkrp_ffma(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,
                 int round, void *ws, cudaStream_t s);
+// Estimated time of a kernel's main loop (us on B200), for the dispatcher.
+double mttkrp_ffma_us(int order, const long *dims, int mode, long R, int round);
+double mttkrp_simt_us(int order, const long *dims, int mode, long R, int round);
 // Small tensors in one launch, plain FP32 (mttkrp_small.cu); no workspace.
 bool mttkrp_small_applies(int order, const long *dims, int mode, long R);
 int mttkrp_small(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,

@@ -5,8 +5,9 @@
 // otherwise the CUDA-core kernel with the same operand rounding
 // (BF16X3/DEFAULT fall back to plain FP32, which is at least as accurate).
 // DEFAULT takes whichever of the two is faster.
-// The CUDA-core kernel of the entry points is mttkrp_ffma.cu's; a CP-ALS
-// plan's sweeps keep mttkrp_simt.cu's (see there).
+// The CUDA-core kernel of the entry points is mttkrp_ffma.cu's, or
+// mttkrp_simt.cu's where the fastest factor has few rows; a CP-ALS plan's
+// sweeps keep mttkrp_simt.cu's throughout (see there).
 #include "kernels.cuh"
 #include "tc_ptx.cuh"
 
@@ -79,6 +80,18 @@ bool small_path(int order, const long *dims, int mode, long R, int precision) {
     return (precision == CUD_PREC_FP32 || precision == CUD_PREC_DEFAULT) && mttkrp_small_applies(order, dims, mode, R);
 }
 
+// A stage of k_mttkrp_ffma ends with a row block of the fastest factor, so with
+// few rows there it is shallow, and k_mttkrp_simt's flat steps can be the faster
+// ones: by the two kernels' estimates (B200, us, FFMA / flat steps: BF16 2 x 2 x
+// 1000 x 1000 R = 8 mode 1 5700 / 1236, 5 x 700 x 700 R = 32 mode 1 58 / 37, 17 x 301 x
+// 301 R = 64 28.8 / 30.7; FP32 2 x 4 x 301 x 101 R = 64 mode 0 188 / 102, mode 1 169 /
+// 476, 7 x 301 x 301 R = 64 18.4 / 18.7).
+bool simt_faster(int order, const long *dims, int mode, long R, int round) {
+    int oth[kMaxOrder];
+    const long rows0 = other_modes(order, dims, mode, oth) ? dims[oth[0]] : 1;
+    return rows0 < 32 && mttkrp_ffma_us(order, dims, mode, R, round) > mttkrp_simt_us(order, dims, mode, R, round);
+}
+
 // CUD_PREC_DEFAULT picks the faster of the tensor cores (BF16x3) and plain
 // FP32, never the less accurate one where they tie.  The tensor cores are
 // faster where the packed-B kernel runs, above 6.5e7 multiply-adds (B200, us a
@@ -98,7 +111,9 @@ bool default_fp32(int order, const long *dims, int mode, long R, int precision) 
 // Sized for both paths, so a call may fall back (e.g. a misaligned X) with
 // the same workspace.
 size_t mttkrp_ws_bytes(int order, const long *dims, int mode, long R, int precision) {
-    size_t b = mttkrp_ffma_ws_bytes(order, dims, mode, R, round_mode(precision));
+    const int round = round_mode(precision);
+    size_t b = simt_faster(order, dims, mode, R, round) ? mttkrp_simt_ws_bytes(order, dims, mode, R, round)
+                                                        : mttkrp_ffma_ws_bytes(order, dims, mode, R, round);
     size_t t = 0;
     if (precision != CUD_PREC_FP32 && mttkrp_tc_query(order, dims, mode, R, precision, &t) == CUD_OK)
         b = std::max(b, t);
@@ -115,7 +130,9 @@ int mttkrp_run(const float *X, int order, const long *dims, const float *const *
             if (st != CUD_ERR_UNSUPPORTED) return st;
         }
     }
-    return mttkrp_ffma(X, order, dims, U, mode, R, out, round_mode(precision), ws, s);
+    const int round = round_mode(precision);
+    return simt_faster(order, dims, mode, R, round) ? mttkrp_simt_rounded(X, order, dims, U, mode, R, out, round, ws, s)
+                                                    : mttkrp_ffma(X, order, dims, U, mode, R, out, round, ws, s);
 }
 
 size_t mttkrp_sweep_ws_bytes(int order, const long *dims, int mode, long R, int precision) {

@@ -513,6 +513,27 @@ int launch_nr(const FfmaPlan &p, const FfmaArgs &a, dim3 grid, cudaStream_t s) {
 
 }  // namespace
 
+// Microseconds that a CTA's stages take on B200, launches aside: fitted to 1048
+// timed modes whose fastest factor has 2 to 24 rows (ranks 1 to 64, orders 2 to
+// 5).  A stage of few kappas costs its barrier, the constant row's gathers and
+// its copies (by the rank lanes, a third of it again for a full tile of rows
+// q, and with 64-bit digits by their number), whatever its depth; the 64-rank
+// tile's final sum takes 5 us.
+double mttkrp_ffma_us(int order, const long *dims, int mode, long R, int round) {
+    static const double kStage[4] = {0.9, 1.5, 1.3, 1.4}, kAnyStage[4] = {2.0, 2.2, 2.3, 2.7};
+    static const double kDepth[4] = {0.0, 0.7, 0.7, 0.8}, kEnd[4] = {1.0, 1.1, 0.7, 4.7};
+    const FfmaPlan p = ffma_plan(order, dims, mode, R, round);
+    const int i = p.NR == 1 ? 0 : p.NR == 2 ? 1 : p.NR == 4 ? 2 : 3;
+    const int tq = p.NR == 1 ? 4 : p.NR == 2 ? 8 : 16;
+    const long ctas = p.qtiles * p.rtiles * p.splits, wave = (tq * p.TR <= 96 ? 3L : 2L) * kNumSMs;
+    int oth[kMaxOrder];
+    const int nf = other_modes(order, dims, mode, oth);
+    const long rows0 = nf ? dims[oth[0]] : 1;
+    const double stage = (p.any ? kAnyStage : kStage)[i] + 0.6 * std::min(dims[mode], (long)FQ) / FQ +
+                         kDepth[i] * std::min(rows0, (long)FK) / FK + (p.any ? 0.3 * std::max(0, nf - 3) : 0.0);
+    return (kEnd[i] + stage * p.chunk) * ((ctas + wave - 1) / wave);
+}
+
 size_t mttkrp_ffma_ws_bytes(int order, const long *dims, int mode, long R, int round) {
     return sizeof(float) * (size_t)ffma_plan(order, dims, mode, R, round).splits * R * dims[mode];
 }

@@ -2,8 +2,9 @@
 // fallback for shapes the tensor-core path does not take.  Native layout, no
 // unfolding, no materialised Khatri-Rao matrix.
 //
-// The MTTKRP entry points run the faster kernel of mttkrp_ffma.cu, which sums
-// a contraction in another order.  A plan's sweeps keep the order of the
+// The MTTKRP entry points run the kernel of mttkrp_ffma.cu, which sums a
+// contraction in another order, except where the fastest factor has few rows
+// (see mttkrp.cu).  A plan's sweeps keep the order of the
 // kernels here, so that their factors stay the same to the bit: a program may
 // set new factors and run on with the plan's old Grams, whose sweeps multiply
 // a difference of rounding without bound until they have caught up (105 x 236
@@ -462,6 +463,16 @@ FfmaPlan ffma_plan(int order, const long *dims, int mode, long R) {
 }
 
 }  // namespace
+
+// Microseconds that a CTA's steps take in k_mttkrp_simt on B200, launches
+// aside (fitted as mttkrp_ffma_us): a step of 16 kappas, its digits by 64-bit
+// divisions, whatever the rank up to 64.
+double mttkrp_simt_us(int order, const long *dims, int mode, long R, int round) {
+    static const double kStep[3] = {4.6, 6.4, 3.5};  // by kind
+    const SimtPlan p = simt_plan(mode_view(order, dims, mode), mode, R, round);
+    const long ctas = p.qtiles * p.rtiles * p.splits, wave = 3L * kNumSMs;
+    return kStep[p.kind] * p.chunk * ((ctas + wave - 1) / wave);
+}
 
 size_t mttkrp_simt_ws_bytes(int order, const long *dims, int mode, long R, int round) {
     ModeView v = mode_view(order, dims, mode);
