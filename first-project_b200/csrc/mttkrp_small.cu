@@ -131,7 +131,13 @@ bool mttkrp_small_applies(int order, const long *dims, int mode, long R) {
         work *= (double)dims[m];
         if (m != mode) K *= (double)dims[m];
     }
-    return R <= 64 && work <= 1e7 && K <= 16384.0;
+    // A CTA computes whole tiles of 4 rows x 8 ranks, and all of its 256 threads
+    // sum them, however short the contraction (us, this kernel / the one that
+    // had the call before it: 10 x 1000 x 1000 R = 1 mode 2 44 / 33, 2 x 6 x 5000 R = 64
+    // mode 2, 10000 tiles over K = 12, 53 / 8, 9 x 5 x 2291 R = 33 mode 2, 2865 tiles, 18 /
+    // 8; 12 x 18 x 932 R = 34 mode 2, 1165 tiles, 9.5 / 9.8).
+    const double tiles = (double)((dims[mode] + SQ - 1) / SQ) * (double)((R + SR - 1) / SR);
+    return R <= 64 && work <= 1e7 && K <= 16384.0 && tiles <= 8.0 * kNumSMs && tiles * (SQ * SR) * K <= 2e7;
 }
 
 int mttkrp_small(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,
