@@ -106,6 +106,7 @@ int mttkrp_ffma(const float *X, int order, const long *dims, const float *const 
 // Estimated time of a kernel's main loop (us on B200), for the dispatcher.
 double mttkrp_ffma_us(int order, const long *dims, int mode, long R, int round);
 double mttkrp_simt_us(int order, const long *dims, int mode, long R, int round);
+double mttkrp_tc_us(int order, const long *dims, int mode, long R, int precision);
 // Small tensors in one launch, plain FP32 (mttkrp_small.cu); no workspace.
 bool mttkrp_small_applies(int order, const long *dims, int mode, long R);
 int mttkrp_small(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,

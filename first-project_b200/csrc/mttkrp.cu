@@ -91,19 +91,32 @@ bool simt_faster(int order, const long *dims, int mode, long R, int round) {
     const long rows0 = other_modes(order, dims, mode, oth) ? dims[oth[0]] : 1;
     return rows0 < 32 && mttkrp_ffma_us(order, dims, mode, R, round) > mttkrp_simt_us(order, dims, mode, R, round);
 }
+double cuda_core_us(int order, const long *dims, int mode, long R, int round) {
+    return simt_faster(order, dims, mode, R, round) ? mttkrp_simt_us(order, dims, mode, R, round)
+                                                    : mttkrp_ffma_us(order, dims, mode, R, round);
+}
 
 // CUD_PREC_DEFAULT picks the faster of the tensor cores (BF16x3) and plain
-// FP32, never the less accurate one where they tie.  The tensor cores are
-// faster where the packed-B kernel runs, above 6.5e7 multiply-adds (B200, us a
-// mode, tensor cores / FP32: 160^3 R = 16 16.5 / 16.5, R = 32 17.0 / 22.0, 128^3
-// R = 32 16.3 / 13.7, R = 64 16.4 / 18.2, 256^3 R = 8 22.9 / 34.2); where the
-// Khatri-Rao rows are built per stage they are the slower ones (200^3 R = 16
-// 52 / 22, R = 64 105 / 48, 500^3 R = 32 704 / 248, 100^4 R = 16 512 / 164).
+// FP32, never the less accurate one where they tie.  Where the packed-B kernel
+// runs, the tensor cores are faster above 8e7 multiply-adds, counting whole
+// tiles of 128 rows, which both kernels compute (B200, us a mode, tensor cores /
+// FP32: 160^3 R = 12 (7.9e7) 14.3 / 13.7, 128^3 R = 32 (6.7e7) 12.1 / 11.3, R = 48
+// (1.0e8) 13.5 / 15.1, 256 x 4 x 256 mode 1 R = 8 (6.7e7) 15.4 / 12.3, R = 32
+// (2.7e8) 18.4 / 21.3, R = 64 16.2 / 34.9).  Where the Khatri-Rao rows are built
+// per stage they mostly are the slower ones, by the kernels' estimates (200^3 R =
+// 16 52 / 22, R = 64 105 / 48, 500^3 R = 32 704 / 248, 100^4 R = 16 512 / 164; but 3 x
+// 256 x 256 x 32 R = 16 mode 2 42 / 72, 2 x 2 x 1000 x 1000 R = 8 mode 3 23 / 61).
 bool default_fp32(int order, const long *dims, int mode, long R, int precision) {
     if (precision != CUD_PREC_DEFAULT) return false;
-    double work = (double)R;
-    for (int m = 0; m < order; m++) work *= (double)dims[m];
-    return work <= 6.5e7 || !mttkrp_tc_packed(order, dims, mode, R, precision);
+    size_t b = 0;
+    if (mttkrp_tc_query(order, dims, mode, R, precision, &b) != CUD_OK) return true;
+    if (mttkrp_tc_packed(order, dims, mode, R, precision)) {
+        double work = (double)R * (double)((dims[mode] + 127) / 128 * 128);
+        for (int m = 0; m < order; m++)
+            if (m != mode) work *= (double)dims[m];
+        return work <= 8e7;
+    }
+    return cuda_core_us(order, dims, mode, R, 0) <= mttkrp_tc_us(order, dims, mode, R, precision);
 }
 
 }  // namespace
