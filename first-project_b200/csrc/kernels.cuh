@@ -141,7 +141,8 @@ int mttkrp_tc(const float *X, int order, const long *dims, const float *const *U
 // one lane each (with the MTTKRP, 100000 x 6 x 6 R = 8, one split: FP64 18 us, 28
 // with 32 outputs a CTA, 78 with 32 lanes; FP32 17, 32 with 8 lanes).
 inline int sum_lanes(int splits, long n) {
-    return splits >= 32 && (n + 31) / 32 < 2L * kNumSMs ? 32 : splits >= 8 ? 8 : 1;
+    if (splits >= 32) return (n + 31) / 32 < 2L * kNumSMs ? 32 : 8;
+    return splits >= 8 && n < 256L * kNumSMs ? 8 : 1;
 }
 __host__ __device__ constexpr int sum_width(int lanes) { return lanes == 1 ? 256 : 32; }
 // The split reduce (mttkrp.cu): out (Q x R, column-major) = the sum of the
