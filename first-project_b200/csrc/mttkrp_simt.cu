@@ -468,9 +468,9 @@ FfmaPlan ffma_plan(int order, const long *dims, int mode, long R) {
 // aside (fitted as mttkrp_ffma_us): a step of 16 kappas, its digits by 64-bit
 // divisions, whatever the rank up to 64.
 double mttkrp_simt_us(int order, const long *dims, int mode, long R, int round) {
-    static const double kStep[3] = {4.6, 6.4, 3.5};  // by kind
+    static const double kStep[3] = {4.6, 3.6, 3.5};  // by kind, of which 1 has registers for two CTAs an SM
     const SimtPlan p = simt_plan(mode_view(order, dims, mode), mode, R, round);
-    const long ctas = p.qtiles * p.rtiles * p.splits, wave = 3L * kNumSMs;
+    const long ctas = p.qtiles * p.rtiles * p.splits, wave = (p.kind == 1 ? 2L : 3L) * kNumSMs;
     return kStep[p.kind] * p.chunk * ((ctas + wave - 1) / wave);
 }
 
