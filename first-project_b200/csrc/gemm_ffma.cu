@@ -355,21 +355,23 @@ __global__ void __launch_bounds__(FT, Tile<kQ, NR, TR>::MINB) k_gemm_ffma(const 
 }
 
 // C(m, n) = the sum over the splits of the dense M x N partials, in
-// FP64 and a fixed order: a CTA owns 32 consecutive outputs, 8 lanes each.
+// FP64 and a fixed order: a CTA owns 256 / ZL consecutive outputs, ZL lanes each.
+template <int ZL>
 __global__ void __launch_bounds__(256) k_gemm_sum(const float *__restrict__ part, int splits, long M, long N, void *C,
                                                   long c_m, long c_n, int f64) {
-    __shared__ double red[8][32];
-    const int o = threadIdx.x & 31, zl = threadIdx.x >> 5;
-    const long e = blockIdx.x * 32L + o, n = M * N;
+    constexpr int OW = 256 / ZL;
+    __shared__ double red[ZL][OW];
+    const int o = threadIdx.x % OW, zl = threadIdx.x / OW;
+    const long e = blockIdx.x * (long)OW + o, n = M * N;
     double sum = 0.0;
     if (e < n) {
 #pragma unroll 8
-        for (int z = zl; z < splits; z += 8) sum += (double)part[(long)z * n + e];
+        for (int z = zl; z < splits; z += ZL) sum += (double)part[(long)z * n + e];
     }
     red[zl][o] = sum;
     __syncthreads();
     if (zl == 0 && e < n) {
-        for (int k = 1; k < 8; k++) sum += red[k][o];
+        for (int k = 1; k < ZL; k++) sum += red[k][o];
         const long j = e / M, i = e - j * M, off = i * c_m + j * c_n;
         if (f64) static_cast<double *>(C)[off] = sum;
         else static_cast<float *>(C)[off] = (float)sum;
@@ -449,6 +451,11 @@ int gemm_ffma(const GemmDesc &d, cudaStream_t s) {
     // (A 4096 x 4096 Gram over K = 64, whose partials pass through memory: 498
     // against 250 us.)
     if (K < (d.out_f64 ? 512 : g.c_n == 1 ? 96 : 64)) return CUD_ERR_UNSUPPORTED;
+    // A stage does not leave its kout: with a short inner contraction the flat
+    // 16-deep slices of the 64 x 64 tile are the faster ones (B200, Gram of mode 1,
+    // us: 2 x 300 x 1000 117 against 50, 5 x 300 x 1000 136 against 116, 7 x 200 x 999 81
+    // against 121).
+    if (g.Kout > 1 && g.Kin < 6) return CUD_ERR_UNSUPPORTED;
     // splits of the contraction for one wave of the resident CTAs, at least
     // four stages each
     long splits = d.splits;
@@ -457,6 +464,15 @@ int gemm_ffma(const GemmDesc &d, cudaStream_t s) {
         const long want = std::max(1L, (tq * TR <= 96 ? 3L : 2L) * kNumSMs / tiles);
         splits = d.batch > 1 ? 1 : std::max(1L, std::min(std::min(want, (g.steps + 3) / 4), 256L));
     }
+    const bool few = tiles * splits < kNumSMs;
+    if (d.splits <= 0 && splits > 1) {
+        // a few CTAs more than SMs double the time: fewer, longer ones then
+        // (B200, Grams of 100^3 by mode, us: 158 and 200 CTAs 28.0 / 25.9 / 26.9, 126 and
+        // 134 with longer ranges 23.2 / 22.6 / 22.3)
+        const long even = kNumSMs / tiles, longer = even > 0 ? (g.steps + even - 1) / even : 0;
+        const long turns = (tiles * splits + kNumSMs - 1) / kNumSMs;
+        if (even > 0 && even < splits && longer < (g.steps + splits - 1) / splits * turns) splits = even;
+    }
     g.chunk = (g.steps + splits - 1) / splits;
     splits = (g.steps + g.chunk - 1) / g.chunk;
     if (g.chunk > 0x7fffffffL || splits > 65535) return CUD_ERR_UNSUPPORTED;
@@ -464,7 +480,23 @@ int gemm_ffma(const GemmDesc &d, cudaStream_t s) {
     // the 64 x 64 tile, whose CTAs are more and wider, is the faster one above
     // 32 columns (B200, TTM of 256 x 256 x 16, mode 0, 32 tiles: J = 64 27
     // against 23 us, J = 32 17 against 23).
-    if (tiles * splits < kNumSMs && NR == 8) return CUD_ERR_UNSUPPORTED;
+    if (few && NR == 8) return CUD_ERR_UNSUPPORTED;
+    // (70^3, 39 tiles over K = 70: J = 32 8.2 against 7.3.)
+    if (tiles * splits < kNumSMs / 3 && NR == 4 && K < 96) return CUD_ERR_UNSUPPORTED;
+    // Above 32 columns the two tiles multiply at the same rate, and the 64 x 64
+    // one spreads over the SMs more evenly; this one gains by rows that fill whole
+    // tiles over a batch and by a long operand that lies along k.  In us per
+    // wave of the SMs, fitted to mode products over K = 64 to 1000 (B200, this tile
+    // / 64 x 64: 1000 x 1000 x 20 mode 1 J = 64 139 / 119, 500 x 64 x 80 mode 1 J = 64 24 / 19,
+    // 200^3 mode 2 J = 64 51 / 45; mode 1 J = 64 52 / 54, J = 200 146 / 184, mode 0 J = 64
+    // 50 / 60, 31 x 77 x 500 mode 1 J = 128 19 / 29).
+    if (NR == 8 && !d.out_f64) {
+        const double turns = (double)((tiles * splits + kNumSMs - 1) / kNumSMs);
+        const double mine = 1.0 + (TR == 8 ? 1.0 : 0.9) * (2.5 + 0.07 * K) * turns;
+        const double old = (double)((d.M + 63) / 64 * ((d.N + 63) / 64) * d.batch) / (2.0 * kNumSMs);
+        const double other = (g.l_r == 1 ? 1.0 : 1.22) * (2.0 + 0.045 * K + (1.5 + 0.07 * K) * old);
+        if (mine > other) return CUD_ERR_UNSUPPORTED;
+    }
     const bool part = d.out_f64 || splits > 1;
     g.C = static_cast<float *>(d.C);
     g.c_z = 0;
@@ -492,7 +524,12 @@ int gemm_ffma(const GemmDesc &d, cudaStream_t s) {
     if (st) return st;
     if (part) {
         const long n = d.M * d.N;
-        k_gemm_sum<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(g.C, (int)splits, d.M, d.N, d.C, d.c_m, d.c_n, d.out_f64);
+        if (sum_lanes((int)splits, n) > 1)
+            k_gemm_sum<8><<<(unsigned)((n + 31) / 32), 256, 0, s>>>(g.C, (int)splits, d.M, d.N, d.C, d.c_m, d.c_n,
+                                                                    d.out_f64);
+        else
+            k_gemm_sum<1><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g.C, (int)splits, d.M, d.N, d.C, d.c_m, d.c_n,
+                                                                      d.out_f64);
         CUD_CHECK_LAUNCH("gemm_ffma reduce");
     }
     return CUD_OK;
