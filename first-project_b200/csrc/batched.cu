@@ -757,7 +757,15 @@ int launch_cfg(const BatchArgs &a, const BatchCfg &c, cudaStream_t s) {
 // 0.86 / 1.06 / 1.55; 1024: 1.59 / 1.63 / 2.00 / -; 2048: 2.90 / 3.19 / 3.93.
 // (Six warps a CTA of 2 x 8 register tiles without clusters: 0.92 ms at 64,
 // 1.28 at 256, 2.0 at 1024, 3.2 at 2048.)
-BatchCfg default_cfg(int n) {
+// Tensors of up to 40000 elements have too little to share: their sweeps are
+// barriers, which a cluster's make longer (B200, ms for 20 sweeps, clusters of 1 /
+// 2 / 4 / 8: 60 tensors of dims 10 to 20 0.98 / 1.07 / 1.15 / 1.64, 200 1.19 / 1.76 /
+// 2.32 / 4.24; dims 16 to 32, 100 tensors 1.42 / 1.41 / 2.06 / 3.17, 300 1.86 / 2.76 /
+// 4.28 / 7.75; dims 24 to 48, 100 tensors 2.93 / 2.55 / 2.74 / 4.33).
+BatchCfg default_cfg(int n, const int *dims) {
+    int largest = 0;
+    for (int t = 0; t < n; t++) largest = std::max(largest, dims[3 * t] * dims[3 * t + 1] * dims[3 * t + 2]);
+    if (largest <= 40000) return {192, 2, 1};
     if (n <= kNumSMs / 2) return {192, 2, 8};
     if (n <= 2 * kNumSMs) return {192, 2, 4};
     if (n <= 6 * kNumSMs) return {192, 2, 2};
@@ -847,9 +855,9 @@ int batched_impl(int ntensors, const long *dims, const long *ranks, const float 
     k_batch_setup<<<std::min((long)ntensors * NORM_PARTS, kNumSMs * 64L), 256, 0, s>>>(a.meta, a.state, ntensors, X, U);
     CUD_CHECK_LAUNCH("batched setup");
 
-    // launch shape from the autotuner (threads per CTA, CTAs per SM, tile rows)
+    // launch shape: the autotuner's (CTAs a tensor), where this class was tuned
     long key = shape_class(ntensors, hd.data(), hr.data());
-    BatchCfg cfg = default_cfg(ntensors);
+    BatchCfg cfg = default_cfg(ntensors, hd.data());
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune.find(key);
@@ -949,9 +957,10 @@ extern "C" int cud_cp_batched_tune(int ntensors, const long *dims, const long *r
     }
     long key = shape_class(ntensors, hd.data(), hr.data());
     // (threads, CTAs per SM, CTAs a tensor): two CTAs of 168 registers a thread
-    // and ~100 KB of shared memory fill an SM
+    // and ~100 KB of shared memory fill an SM, so the first two, which the
+    // caller is told, are the same throughout
     const std::vector<BatchCfg> cand = {{192, 2, 1}, {192, 2, 2}, {192, 2, 4}, {192, 2, 8}};
-    BatchCfg bestc = default_cfg(ntensors);
+    BatchCfg bestc = cand[0];
     cudaStream_t s = as_stream(stream);
     cudaEvent_t e0, e1;
     CUD_CHECK(cudaEventCreate(&e0));

@@ -333,12 +333,12 @@ int cud_cp_als_batched_target(int ntensors, const long *dims, const long *ranks,
                               const cud_cp_options *opt, const double *target_fits, double *fits, int *sweeps,
                               int *kernel_launches, void *stream);
 
-/* Extension: autotunes the batched sweep's launch shape (threads per CTA,
- * CTAs per SM, and the rows of the MTTKRP register tile, 2 or 4) for this
- * batch's shape class by timing two sweeps per candidate; U_scratch is a
- * copy of the factors (overwritten).  The choice is cached per shape class
- * and used by later cud_cp_als_batched calls; threads and ctas_per_sm
- * report the first two. */
+/* Extension: autotunes the batched sweep's launch shape (the number of CTAs
+ * that share a tensor) for this batch's shape class by timing two sweeps per
+ * candidate; U_scratch is a copy of the factors (overwritten).  The choice is
+ * cached per shape class and used by later cud_cp_als_batched calls, whose
+ * results do not depend on it.  threads and ctas_per_sm report the threads of
+ * a CTA and the CTAs of an SM, the same for every choice (192 and 2). */
 int cud_cp_batched_tune(int ntensors, const long *dims, const long *ranks, const float *X,
                         const long *x_offsets, float *U_scratch, const long *u_offsets, int *threads,
                         int *ctas_per_sm, void *stream);
