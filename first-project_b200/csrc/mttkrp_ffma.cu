@@ -81,10 +81,6 @@ __device__ __forceinline__ void copy4(uint32_t dst, const float *src) {
 __device__ __forceinline__ void copy16(uint32_t dst, const float *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
-__device__ __forceinline__ void zero4(uint32_t dst) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst), "f"(0.f)); }
-__device__ __forceinline__ void zero16(uint32_t dst) {
-    asm volatile("st.shared.v4.f32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "f"(0.f));
-}
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 dup2(float x) {
@@ -214,10 +210,6 @@ __global__ void __launch_bounds__(FT, Tile<kQ, NR, TR>::MINB) k_mttkrp_ffma(cons
                 if constexpr (kVec) copy16(d + place(i), p);
                 else copy4(d + place(i), p);
             }
-            if (kQ == 1 && ck >= kc) {  // read in groups of 4 kappas
-#pragma unroll 4
-                for (int i = 0; i < NC; i++) zero16(d + place(i));
-            }
         }
         const uint32_t bd = bdst + (uint32_t)slot * (4u * BF);
         const I row = lj * FK + lane;
@@ -229,7 +221,6 @@ __global__ void __launch_bounds__(FT, Tile<kQ, NR, TR>::MINB) k_mttkrp_ffma(cons
             const uint32_t o = bd + 4u * ((j / 4) * (NR * 4) + l * 4 + (j & 3));
             const I r = (I)min(r0 + c, a.R - 1);
             if (lane < kc) copy4(o, a.U[0] + (row + r * (I)rows0));
-            else zero4(o);
         }
         // the next stage
         lj++;
@@ -368,7 +359,8 @@ __global__ void __launch_bounds__(FT, Tile<kQ, NR, TR>::MINB) k_mttkrp_ffma(cons
                 }
             }
         } else {
-            // the warp's groups of 4 kappas: wk, wk + WK, .. (zeros past kc)
+            // the warp's groups of 4 kappas: wk, wk + WK, .. (kc is a multiple of 4
+            // here: whole 16-byte copies of a row block)
             const float *A = Xring + slot * AF + qrow(0) * LDK + 4 * wk;
             const float *B = Bring + slot * BF + 4 * rl + 4 * wk * T::LDB;
 #pragma unroll 1
