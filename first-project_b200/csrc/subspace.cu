@@ -866,10 +866,13 @@ __device__ __forceinline__ void run_send(cg::cluster_group &cl, const RunLayout 
 }
 
 // state (pinned host memory): 1 converged, 2 not within max_iters, 3 a rank-
-// deficient iterate; U is written in the first case only.
+// deficient iterate; U is written in the first case only.  products: G V or
+// G^2 V a step, and two or one more steps once the tolerance is met -- the steps
+// of the path that had the call before this kernel (see top_eigvecs_run), so
+// that the vectors keep their signs, which are the iterate's.
 template <int NT>
 __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
-    k_si_run_cl(const double *__restrict__ Gm, long n, int r, const float *U0, float *U, int max_iters,
+    k_si_run_cl(const double *__restrict__ Gm, long n, int r, const float *U0, float *U, int max_iters, int products,
                 volatile int *state) {
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) double smc[];
@@ -914,13 +917,18 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
             verdict = 2;
             break;
         }
-        // two products per orthonormalisation (G^2 V): the columns' condition
-        // grows by (lambda_1 / lambda_r)^2 per step, well inside CholQR2's range
-        run_apply<NT>(L, G, va, C, yb);
-        for (int e = threadIdx.x; e < (L.kp - (int)n) * L.ldv; e += CL_T) vb[n * L.ldv + e] = 0.0;
-        run_send<NT>(cl, L, yb, nl, i0, vb);
-        cl.sync();
-        run_apply<NT>(L, G, vb, C, ya);
+        if (products == 2) {
+            // two products per orthonormalisation (G^2 V): the columns' condition
+            // grows by (lambda_1 / lambda_r)^2 per step, well inside CholQR2's range
+            run_apply<NT>(L, G, va, C, yb);
+            for (int e = threadIdx.x; e < (L.kp - (int)n) * L.ldv; e += CL_T) vb[n * L.ldv + e] = 0.0;
+            run_send<NT>(cl, L, yb, nl, i0, vb);
+            cl.sync();
+            run_apply<NT>(L, G, vb, C, ya);
+        } else {
+            run_apply<NT>(L, G, va, C, ya);
+            cl.sync();  // the gap's buffer has been read by every peer
+        }
         if (!cl_orth(cl, ya, yb, nl, r, red, gp, C, T, pub, dsh)) {
             verdict = 3;
             break;
@@ -936,8 +944,9 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T)
         cl.sync();
         cl_sum(cl, red, r, false, C);
         const double gap = cl_gap(C, r, wred);
-        // one more step after the gap first falls below the tolerance
-        if (extra < 0 && gap < 1e-13 * (double)r) extra = 1;
+        // one more step (two of one product) after the gap first falls below the
+        // tolerance
+        if (extra < 0 && gap < 1e-13 * (double)r) extra = 3 - products;
         if (extra >= 0 && extra-- == 0) verdict = 1;
     }
     if (verdict == 1) {
@@ -1125,9 +1134,12 @@ size_t subspace_ws_doubles(long n, long r) { return 3 * (size_t)n * r + 8; }  //
 
 // The whole iteration in one launch of a cluster (k_si_run_cl).
 // CUD_ERR_UNSUPPORTED when its shared memory or the cluster does not fit.
+// Steps of two products where ws_doubles would hold top_eigvecs_fast's partial
+// products (it needs no workspace itself), of one where the general loop below
+// would run.
 template <int NT>
-static int top_eigvecs_run(const double *G, long n, long r, float *U, int max_iters, cudaStream_t s,
-                           const float *U0) {
+static int top_eigvecs_run(const double *G, long n, long r, float *U, size_t ws_doubles, int max_iters,
+                           cudaStream_t s, const float *U0) {
     const size_t smem = run_layout(n, NT).total * sizeof(double);
     if (smem > RUN_SMEM_MAX) return CUD_ERR_UNSUPPORTED;
     int dev = 0;
@@ -1150,7 +1162,8 @@ static int top_eigvecs_run(const double *G, long n, long r, float *U, int max_it
     if (!h) return CUD_ERR_NO_MEMORY;
     volatile int *state = reinterpret_cast<volatile int *>(h);
     *state = 0;
-    k_si_run_cl<NT><<<CL_N, CL_T, smem, s>>>(G, n, (int)r, U0, U, max_iters, state);
+    const int products = ws_doubles >= 4 * (size_t)n * r + 8 ? 2 : 1;
+    k_si_run_cl<NT><<<CL_N, CL_T, smem, s>>>(G, n, (int)r, U0, U, max_iters, products, state);
     CUD_CHECK_LAUNCH("subspace iteration");
     CUD_CHECK(cudaStreamSynchronize(s));
     return *state == 1 ? CUD_OK : CUD_ERR_NOT_CONVERGED;
@@ -1239,10 +1252,10 @@ static int top_eigvecs_fast(const double *G, long n, long r, float *U, double *w
 static int subspace_run(const double *G, long n, long r, float *U, double *ws, size_t ws_doubles, int max_iters,
                         cudaStream_t s, const float *U0) {
     if (r <= SI_FR) {
-        const int st = r <= 8    ? top_eigvecs_run<1>(G, n, r, U, max_iters, s, U0)
-                       : r <= 16 ? top_eigvecs_run<2>(G, n, r, U, max_iters, s, U0)
-                       : r <= 24 ? top_eigvecs_run<3>(G, n, r, U, max_iters, s, U0)
-                                 : top_eigvecs_run<4>(G, n, r, U, max_iters, s, U0);
+        const int st = r <= 8    ? top_eigvecs_run<1>(G, n, r, U, ws_doubles, max_iters, s, U0)
+                       : r <= 16 ? top_eigvecs_run<2>(G, n, r, U, ws_doubles, max_iters, s, U0)
+                       : r <= 24 ? top_eigvecs_run<3>(G, n, r, U, ws_doubles, max_iters, s, U0)
+                                 : top_eigvecs_run<4>(G, n, r, U, ws_doubles, max_iters, s, U0);
         if (st != CUD_ERR_UNSUPPORTED) return st;
     }
     if (r <= SI_FR && n <= 2048 && cl_layout(n).total * sizeof(double) <= CL_SMEM_MAX) {
