@@ -98,11 +98,13 @@ double cuda_core_us(int order, const long *dims, int mode, long R, int round) {
 
 // CUD_PREC_DEFAULT picks the faster of the tensor cores (BF16x3) and plain
 // FP32, never the less accurate one where they tie.  Where the packed-B kernel
-// runs, the tensor cores are faster above 8e7 multiply-adds, counting whole
-// tiles of 128 rows, which both kernels compute (B200, us a mode, tensor cores /
-// FP32: 160^3 R = 12 (7.9e7) 14.3 / 13.7, 128^3 R = 32 (6.7e7) 12.1 / 11.3, R = 48
+// runs, the tensor cores are faster above 8e7 multiply-adds -- 6e7 for the ranks
+// whose FP32 tile is the less efficient one, 13 to 24 and above 64 --, counting
+// whole tiles of 128 rows, which both kernels compute (B200, us a mode, tensor
+// cores / FP32: 160^3 R = 12 (7.9e7) 14.3 / 13.7, 128^3 R = 32 (6.7e7) 12.1 / 11.3, R = 48
 // (1.0e8) 13.5 / 15.1, 256 x 4 x 256 mode 1 R = 8 (6.7e7) 15.4 / 12.3, R = 32
-// (2.7e8) 18.4 / 21.3, R = 64 16.2 / 34.9).  Where the Khatri-Rao rows are built
+// (2.7e8) 18.4 / 21.3, R = 64 16.2 / 34.9; 32^4 R = 17 (7.1e7) 12.1 / 14.2, 160 x 32 x 32 R =
+// 122 (8.0e7) 13.0 / 15.3).  Where the Khatri-Rao rows are built
 // per stage they mostly are the slower ones, by the kernels' estimates (200^3 R =
 // 16 52 / 22, R = 64 105 / 48, 500^3 R = 32 704 / 248, 100^4 R = 16 512 / 164; but 3 x
 // 256 x 256 x 32 R = 16 mode 2 42 / 72, 2 x 2 x 1000 x 1000 R = 8 mode 3 23 / 61).
@@ -114,7 +116,7 @@ bool default_fp32(int order, const long *dims, int mode, long R, int precision) 
         double work = (double)R * (double)((dims[mode] + 127) / 128 * 128);
         for (int m = 0; m < order; m++)
             if (m != mode) work *= (double)dims[m];
-        return work <= 8e7;
+        return work <= ((R > 12 && R <= 24) || R > 64 ? 6e7 : 8e7);
     }
     return cuda_core_us(order, dims, mode, R, 0) <= mttkrp_tc_us(order, dims, mode, R, precision);
 }

@@ -521,7 +521,9 @@ double mttkrp_ffma_us(int order, const long *dims, int mode, long R, int round) 
     int oth[kMaxOrder];
     const int nf = other_modes(order, dims, mode, oth);
     const long rows0 = nf ? dims[oth[0]] : 1;
-    const double stage = (p.any ? kAnyStage : kStage)[i] + 0.6 * std::min(dims[mode], (long)FQ) / FQ +
+    // (the 64-rank tile's figure is for two CTAs an SM; narrower ones run three)
+    const double crowd = i == 3 && tq * p.TR <= 96 ? 1.5 : 1.0;
+    const double stage = (p.any ? kAnyStage : kStage)[i] * crowd + 0.6 * std::min(dims[mode], (long)FQ) / FQ +
                          kDepth[i] * std::min(rows0, (long)FK) / FK + (p.any ? 0.3 * std::max(0, nf - 3) : 0.0);
     return (kEnd[i] + stage * p.chunk) * ((ctas + wave - 1) / wave);
 }

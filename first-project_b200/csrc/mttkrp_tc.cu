@@ -1372,7 +1372,9 @@ double mttkrp_tc_us(int order, const long *dims, int mode, long R, int precision
     if (!tc_plan(order, dims, mode, R, precision, p)) return 0.0;
     const int i = R <= 8 ? 0 : R <= 16 ? 1 : R <= 32 ? 2 : 3;
     const long ctas = p.qtiles * p.splits, wave = (long)p.ctas_per_sm * kNumSMs;
-    const double wide = R > 64 ? R / 64.0 : 1.0;
+    // above 64 ranks by the rank, and a CTA has the SM to itself: 8 x 24 x 64 x 296 x 8
+    // R = 71 mode 4, 779 stages, 3670
+    const double wide = (R > 64 ? R / 64.0 : 1.0) * (p.ctas_per_sm == 1 ? 0.5 : 1.0);
     return (kEnd[i] + kStage[i] * wide * p.chunk) * ((ctas + wave - 1) / wave);
 }
 
