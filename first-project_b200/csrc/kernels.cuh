@@ -53,7 +53,7 @@ inline ModeView mode_view(int order, const long *dims, int mode) {
 constexpr int kMaxOrder = 8;
 
 // BF16 tensor-core GEMM with fused epilogue (gemm_tc.cu); ws holds
-// gemm_tc_ws_bytes (split-contraction partials + error flag).
+// gemm_tc_ws_bytes (split-contraction partials).
 using GemmEpi = cud_gemm_epilogue;
 size_t gemm_tc_ws_bytes(long M, long N, long K);
 int gemm_tc_bf16(const __nv_bfloat16 *A, long lda, const __nv_bfloat16 *B, long ldb, long M, long N, long K,
@@ -69,7 +69,8 @@ size_t subspace_ws_doubles(long n, long r);
 int top_eigvecs_subspace(const double *G, long n, long r, float *U, double *ws, size_t ws_doubles, int max_iters,
                          cudaStream_t s, const float *U0 = nullptr);
 
-// ||X - [[U]]||^2 and ||X||^2 into out2[0..1] (device, FP64), one pass
+// ||X - [[U]]||^2 and ||X||^2 into out2[0..1] (FP64, device or pinned host
+// memory), one pass
 // over X (residual.cu); ws holds cp_residual_ws_bytes.
 size_t cp_residual_ws_bytes(int order, const long *dims);
 int cp_residual(const float *X, int order, const long *dims, const float *const *U, long R, double *out2,
@@ -98,7 +99,7 @@ inline int other_modes(int order, const long *dims, int mode, int (&out)[kMaxOrd
 // MTTKRP kernels take an explicit device workspace (split-contraction
 // partials), so a captured CUDA graph can own its memory.
 //
-// CUDA-core path (mttkrp_ffma.cu): FP32 FMA; with round = 1 (FP16) or 2
+// CUDA-core path (mttkrp_ffma.cu, or mttkrp_simt.cu below): FP32 FMA; with round = 1 (FP16) or 2
 // (BF16) the operands -- X and each formed KR row -- are rounded first.
 size_t mttkrp_ffma_ws_bytes(int order, const long *dims, int mode, long R, int round);
 int mttkrp_ffma(const float *X, int order, const long *dims, const float *const *U, int mode, long R, float *out,
