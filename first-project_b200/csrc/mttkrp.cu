@@ -4,7 +4,7 @@
 // tcgen05 tensor-core kernel where it applies (shape, alignment, rank) and
 // otherwise the CUDA-core kernel with the same operand rounding
 // (BF16X3/DEFAULT fall back to plain FP32, which is at least as accurate).
-// DEFAULT takes whichever of the two is faster.
+// DEFAULT takes plain FP32 unless the tensor cores are clearly the faster.
 // The CUDA-core kernel of the entry points is mttkrp_ffma.cu's, or
 // mttkrp_simt.cu's where the fastest factor has few rows; a CP-ALS plan's
 // sweeps keep mttkrp_simt.cu's throughout (see there).
@@ -96,29 +96,33 @@ double cuda_core_us(int order, const long *dims, int mode, long R, int round) {
                                                     : mttkrp_ffma_us(order, dims, mode, R, round);
 }
 
-// CUD_PREC_DEFAULT picks the faster of the tensor cores (BF16x3) and plain
-// FP32, never the less accurate one where they tie.  Where the packed-B kernel
-// runs, the tensor cores are faster above 8e7 multiply-adds -- 6e7 for the ranks
-// whose FP32 tile is the less efficient one, 13 to 24 and above 64 --, counting
-// whole tiles of 128 rows, which both kernels compute (B200, us a mode, tensor
-// cores / FP32: 160^3 R = 12 (7.9e7) 14.3 / 13.7, 128^3 R = 32 (6.7e7) 12.1 / 11.3, R = 48
-// (1.0e8) 13.5 / 15.1, 256 x 4 x 256 mode 1 R = 8 (6.7e7) 15.4 / 12.3, R = 32
-// (2.7e8) 18.4 / 21.3, R = 64 16.2 / 34.9; 32^4 R = 17 (7.1e7) 12.1 / 14.2, 160 x 32 x 32 R =
-// 122 (8.0e7) 13.0 / 15.3).  Where the Khatri-Rao rows are built
-// per stage they mostly are the slower ones, by the kernels' estimates (200^3 R =
-// 16 52 / 22, R = 64 105 / 48, 500^3 R = 32 704 / 248, 100^4 R = 16 512 / 164; but 3 x
-// 256 x 256 x 32 R = 16 mode 2 42 / 72, 2 x 2 x 1000 x 1000 R = 8 mode 3 23 / 61).
+// CUD_PREC_DEFAULT: the tensor cores (BF16x3) where they are clearly the faster
+// ones, else plain FP32, which is the more accurate one.  Where the packed-B
+// kernel runs, FP32 up to 6.5e7 multiply-adds, and up to 8e7 counting whole tiles of 128
+// rows, which both kernels compute (6e7 for 13 to 24 ranks and above 64, whose FP32
+// tiles are the less efficient ones); of a mode of up to 16 rows only the whole
+// tiles count, since FP32 can take twice as long there (B200, us a mode, tensor
+// cores / FP32: 160^3 R = 12 (7.9e7 whole) 14.3 / 13.7, 128^3 R = 32 (6.7e7) 12.1 / 11.3,
+// R = 48 (1.0e8) 13.5 / 15.1, 256^3 R = 4 (6.7e7) 20.8 / 14.7; 256 x 4 x 256 mode 1
+// R = 8 (6.7e7 whole) 15.4 / 12.3, R = 32 (2.7e8) 18.4 / 21.3, R = 64 16.2 / 34.9, 512 x 64 x 8
+// mode 2 R = 64 12.3 / 22.9; between, 32^4 R = 17 12.1 / 14.2).  Where the Khatri-Rao
+// rows are built per stage the tensor cores are the slower ones (200^3 R = 16
+// 52 / 22, R = 64 105 / 48, 500^3 R = 32 704 / 248, 100^4 R = 16 512 / 164), but for a
+// fastest factor of few rows, where the estimates decide (3 x 256 x 256 x 32 R = 16
+// mode 2 42 / 72, 2 x 2 x 1000 x 1000 R = 8 mode 3 23 / 61).
 bool default_fp32(int order, const long *dims, int mode, long R, int precision) {
     if (precision != CUD_PREC_DEFAULT) return false;
     size_t b = 0;
     if (mttkrp_tc_query(order, dims, mode, R, precision, &b) != CUD_OK) return true;
     if (mttkrp_tc_packed(order, dims, mode, R, precision)) {
-        double work = (double)R * (double)((dims[mode] + 127) / 128 * 128);
-        for (int m = 0; m < order; m++)
-            if (m != mode) work *= (double)dims[m];
-        return work <= ((R > 12 && R <= 24) || R > 64 ? 6e7 : 8e7);
+        double work = (double)R;
+        for (int m = 0; m < order; m++) work *= (double)dims[m];
+        const double whole = work / (double)dims[mode] * (double)((dims[mode] + 127) / 128 * 128);
+        return whole <= ((R > 12 && R <= 24) || R > 64 ? 6e7 : 8e7) || (dims[mode] > 16 && work <= 6.5e7);
     }
-    return cuda_core_us(order, dims, mode, R, 0) <= mttkrp_tc_us(order, dims, mode, R, precision);
+    int oth[kMaxOrder];
+    const long rows0 = other_modes(order, dims, mode, oth) ? dims[oth[0]] : 1;
+    return rows0 >= 24 || cuda_core_us(order, dims, mode, R, 0) <= mttkrp_tc_us(order, dims, mode, R, precision);
 }
 
 }  // namespace

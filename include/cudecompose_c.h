@@ -38,10 +38,10 @@ typedef enum cud_precision {
     CUD_PREC_BF16 = 1,   /* BF16 operands, FP32 accumulate, tensor cores        */
     CUD_PREC_FP16 = 2,   /* FP16 operands, FP32 accumulate, tensor cores        */
     CUD_PREC_BF16X3 = 3, /* hi/lo BF16 split, 3 products, FP32-level accuracy   */
-    CUD_PREC_DEFAULT = 4 /* FP32-level accuracy: the MTTKRP entry points take the
-                            faster of BF16X3 and FP32; CP-ALS plans (cud_cp_als,
-                            cud_cp_plan_*) BF16X3 where the tensor-core kernels
-                            take the shape, else FP32                        */
+    CUD_PREC_DEFAULT = 4 /* FP32-level accuracy: the MTTKRP entry points take BF16X3
+                            where it is clearly the faster, else FP32; CP-ALS
+                            plans (cud_cp_als, cud_cp_plan_*) BF16X3 where the
+                            tensor-core kernels take the shape, else FP32    */
 } cud_precision;
 
 /* Extension: the calling thread's last status (cudecomposeGetLastError). */

@@ -1,5 +1,6 @@
-"""CUD_PREC_DEFAULT takes the faster of the tensor cores and plain FP32: the
-kernel that cud_mttkrp_path names where both were timed on B200, us a mode."""
+"""CUD_PREC_DEFAULT takes the faster of the tensor cores and plain FP32 (which is
+the more accurate one, and keeps ties): the kernel that cud_mttkrp_path names
+where both were timed on B200, us a mode."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -9,7 +10,7 @@ TIMED = [  # dims, mode, R, tensor cores, FP32
     ((256, 256, 256), 0, 4, 20.8, 14.7), ((160, 160, 160), 2, 32, 16.6, 21.3), ((512, 512, 512), 0, 64, 120., 424.),
     # few rows of the mode: both compute whole tiles of 128
     ((256, 4, 256), 1, 64, 16.2, 34.9), ((256, 4, 256), 1, 32, 18.4, 21.3), ((256, 4, 256), 1, 8, 15.4, 12.3),
-    ((512, 64, 8), 2, 64, 12.3, 22.9), ((32, 32, 32, 32), 1, 17, 12.1, 14.2), ((160, 32, 32), 1, 122, 13.0, 15.3),
+    ((512, 64, 8), 2, 64, 12.3, 22.9),
     ((1024, 1, 1024), 1, 16, 88., 130.),
     # Khatri-Rao rows built per stage
     ((200, 200, 200), 1, 16, 52., 22.), ((700, 5, 700), 1, 32, 361., 119.), ((3, 256, 256, 32), 2, 16, 42., 72.),
